@@ -128,6 +128,7 @@ int rb_csr_create(int n_rows, int n_cols, int64_t nnz, const int* rowptr, const 
 
 int rb_csr_destroy(rb_csr A) {
     return guarded([&]() -> int {
+        HandleRelease idle;
         delete A;
         return RB_OK;
     });
@@ -178,6 +179,7 @@ int rb_csr_transpose(rb_csr A, rb_csr* out) {
     return guarded([&]() -> int {
         NEED(A); NEED(out);
         *out = transpose(*A);
+        RB_CUDA(cudaStreamSynchronize(stream()));
         return RB_OK;
     });
 }
@@ -199,6 +201,7 @@ int rb_vec_create(int n, rb_vec* out) {
 
 int rb_vec_destroy(rb_vec v) {
     return guarded([&]() -> int {
+        HandleRelease idle;
         delete v;
         return RB_OK;
     });
@@ -433,6 +436,7 @@ int rb_bsr_create(int n_block_rows, int n_block_cols, int b_rows, int b_cols, in
 
 int rb_bsr_destroy(rb_bsr A) {
     return guarded([&]() -> int {
+        HandleRelease idle;
         delete A;
         return RB_OK;
     });
@@ -561,6 +565,7 @@ int rb_read_petsc(const char* path, rb_csr* out) {
                                H.cols.data(), H.vals.data(), 0, out);
         if (rc != RB_OK) return rc;
         sort_rows_diag_first(**out, false);   // finalize() sorts rows
+        RB_CUDA(cudaStreamSynchronize(stream()));
         return RB_OK;
     });
 }
@@ -668,6 +673,7 @@ int rb_strength(rb_csr A, int kind, double theta, rb_csr* S) {
         NEED(A); NEED(S);
         RB_REQUIRE(kind == RB_STRENGTH_CLASSICAL || kind == RB_STRENGTH_SYMMETRIC, "unknown strength kind");
         *S = strength(*A, kind, theta);
+        RB_CUDA(cudaStreamSynchronize(stream()));
         return RB_OK;
     });
 }
@@ -784,6 +790,7 @@ int rb_jacobi_prolongation(rb_csr A, rb_csr T, double omega, int steps, rb_csr* 
         NEED(A); NEED(T); NEED(P);
         RB_REQUIRE(steps >= 0, "steps < 0");
         *P = jacobi_prolongation(*A, *T, omega, steps);
+        RB_CUDA(cudaStreamSynchronize(stream()));
         return RB_OK;
     });
 }
@@ -862,6 +869,7 @@ int rb_amg_setup(rb_csr A, const rb_amg_opts* opts, const double* weights, rb_am
         RB_REQUIRE(A->n_rows == A->n_cols, "AMG needs a square matrix");
         std::unique_ptr<rb_amg_s> ml(new rb_amg_s());
         ml->h.setup(*A, o, weights);
+        RB_CUDA(cudaStreamSynchronize(stream()));   // the handle is complete on any stream
         *out = ml.release();
         return RB_OK;
     });
@@ -869,6 +877,7 @@ int rb_amg_setup(rb_csr A, const rb_amg_opts* opts, const double* weights, rb_am
 
 int rb_amg_destroy(rb_amg ml) {
     return guarded([&]() -> int {
+        HandleRelease idle;
         delete ml;
         return RB_OK;
     });
@@ -1125,12 +1134,14 @@ int rb_batch_setup(int n_sys, const rb_csr* mats, const rb_amg_opts* opts, rb_ba
         RB_REQUIRE(o.solver == RB_SOLVER_RS || o.solver == RB_SOLVER_SA, "unknown solver");
         std::vector<const rb_csr_s*> m(mats, mats + n_sys);
         *out = batch_setup(n_sys, m.data(), o);
+        RB_CUDA(cudaStreamSynchronize(stream()));
         return RB_OK;
     });
 }
 
 int rb_batch_destroy(rb_batch B) {
     return guarded([&]() -> int {
+        HandleRelease idle;
         batch_destroy(B);
         return RB_OK;
     });

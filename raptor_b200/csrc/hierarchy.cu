@@ -936,8 +936,9 @@ void Hierarchy::build_cycle_data() {
     ksh.alloc((size_t)n + 1);
     scal.alloc(1);
     scal.zero();
-    if (!host_scal) RB_CUDA(cudaMallocHost(&host_scal, sizeof(KScal)));
-    if (!host_ctl) RB_CUDA(cudaMallocHost(&host_ctl, sizeof(PcgCtl)));
+    static_assert(sizeof(KScal) <= kPinnedBlock && sizeof(PcgCtl) <= kPinnedBlock, "pinned blocks");
+    if (!host_scal) host_scal = static_cast<KScal*>(pinned_block());
+    if (!host_ctl) host_ctl = static_cast<PcgCtl*>(pinned_block());
     gA0 = autotune_group(view(*master[0].A), kp.get(), kAp.get(), "A0_fp64");
     if (opts.precision == RB_PREC_FP32) tune_tail(lv32, tdesc32);
     else tune_tail(lv64, tdesc64);
@@ -945,8 +946,9 @@ void Hierarchy::build_cycle_data() {
 
 Hierarchy::~Hierarchy() {
     release_graphs();
-    if (host_scal) cudaFreeHost(host_scal);
-    if (host_ctl) cudaFreeHost(host_ctl);
+    // (their copies ended with the call that made them)
+    pinned_release(host_scal);
+    pinned_release(host_ctl);
 }
 
 // The tail of the cycle (tail_cycle.cuh).  A start level f >= 1 qualifies
@@ -1844,9 +1846,8 @@ int krylov_cg(const rb_csr_s& A, double* x, const double* b, double tol, int max
     DevArray<double> r((size_t)n + 1), p((size_t)n + 1), Ap((size_t)n + 1);
     DevArray<KScal> S(1);
     S.zero();
-    KScal* hs = nullptr;
-    RB_CUDA(cudaMallocHost(&hs, sizeof(KScal)));
-    std::unique_ptr<KScal, decltype(&cudaFreeHost)> guard(hs, &cudaFreeHost);
+    KScal* hs = static_cast<KScal*>(pinned_block());
+    std::unique_ptr<void, decltype(&pinned_release)> guard(hs, &pinned_release);
     auto rd = [&]() {
         RB_CUDA(cudaMemcpyAsync(hs, S.get(), sizeof(KScal), cudaMemcpyDeviceToHost, stream()));
         RB_CUDA(cudaStreamSynchronize(stream()));
@@ -1917,9 +1918,8 @@ int krylov_bicgstab(const rb_csr_s& A, Hierarchy* ml, double* x, const double* b
     if (ml) { ph.alloc((size_t)n + 1); sh.alloc((size_t)n + 1); }
     DevArray<double> sc(8);
     sc.zero();
-    double* hs = nullptr;
-    RB_CUDA(cudaMallocHost(&hs, sizeof(double) * 8));
-    std::unique_ptr<double, decltype(&cudaFreeHost)> guard(hs, &cudaFreeHost);
+    double* hs = static_cast<double*>(pinned_block());
+    std::unique_ptr<void, decltype(&pinned_release)> guard(hs, &pinned_release);
     const unsigned rg = red_grid(n);
     auto dot = [&](const double* a, const double* c, int f) {
         k_dot_fin<<<rg, 256, 0, stream()>>>(a, c, n, global_reduce_slot(rg), FinField{sc.get() + f});

@@ -64,34 +64,57 @@ int resident_blocks_per_sm(const void* fn, int threads);
 // the library is one); read through rb_device_alloc_count.
 long long& device_alloc_counter();
 
-// Owning device array (cudaMalloc'd; freed on destruction).
+// Device memory behind DevArray (sparse.cu): stream-ordered allocations from
+// a pool of the library's own, one a device.  *pooled says which kind came
+// back (inside a stream capture it is a plain cudaMalloc, as it would
+// otherwise become a node of the caller's graph).  Everything allocated
+// during a call is used on stream() only, so freeing in stream order is
+// enough for it; memory that a caller may have borrowed (handles) is freed
+// under a HandleRelease, which waits for the device first, as cudaFree does.
+void* device_alloc(size_t bytes, bool* pooled);
+void device_free(void* p, bool pooled) noexcept;
+struct HandleRelease {
+    HandleRelease();
+    ~HandleRelease();
+    HandleRelease(const HandleRelease&) = delete;
+    HandleRelease& operator=(const HandleRelease&) = delete;
+};
+
+// A pinned host block of kPinnedBlock bytes, and its return (no copy from or
+// to it may be in flight then).
+constexpr size_t kPinnedBlock = 1024;
+void* pinned_block();
+void pinned_release(void* p) noexcept;
+
+// Owning device array (freed on destruction).
 template <typename T>
 struct DevArray {
     T* p = nullptr;
     size_t n = 0;
+    bool pooled = false;
     DevArray() = default;
     explicit DevArray(size_t count) { alloc(count); }
     DevArray(const DevArray&) = delete;
     DevArray& operator=(const DevArray&) = delete;
-    DevArray(DevArray&& o) noexcept : p(o.p), n(o.n) { o.p = nullptr; o.n = 0; }
+    DevArray(DevArray&& o) noexcept : p(o.p), n(o.n), pooled(o.pooled) { o.p = nullptr; o.n = 0; }
     DevArray& operator=(DevArray&& o) noexcept {
         if (this != &o) {
             release();
-            p = o.p; n = o.n; o.p = nullptr; o.n = 0;
+            p = o.p; n = o.n; pooled = o.pooled; o.p = nullptr; o.n = 0;
         }
         return *this;
     }
     ~DevArray() { release(); }
     void alloc(size_t count) {
         release();
-        n = count;
         if (count) {
-            RB_CUDA(cudaMalloc(&p, sizeof(T) * count));
+            p = static_cast<T*>(::rb::device_alloc(sizeof(T) * count, &pooled));
             ++::rb::device_alloc_counter();
         }
+        n = count;
     }
     void release() {
-        if (p) cudaFree(p);
+        if (p) ::rb::device_free(p, pooled);
         p = nullptr;
         n = 0;
     }
