@@ -51,9 +51,13 @@ void set_stream(cudaStream_t s) { g_stream = s ? s : nullptr; }
 // adjoint solve 37.0 -> 14.0 ms).  The pool keeps at most kPoolKeep bytes
 // of freed memory: the driver gives back what is above at every
 // synchronisation, and an allocation that fails gives back the rest and
-// tries once more.
+// tries once more.  Arrays of kPoolLargest and more stay with cudaMalloc:
+// pooled, the gigabytes a large hierarchy frees are unmapped at the next
+// synchronisation, wherever it falls (a 192^3 setup 700 -> 1720 ms and the
+// first solve after it 10.8 -> 380 ms; with the limit 606 ms and as before).
 namespace {
-constexpr unsigned long long kPoolKeep = 1ull << 30;
+constexpr unsigned long long kPoolKeep = 2ull << 30;
+constexpr size_t kPoolLargest = (size_t)64 << 20;
 constexpr int kMaxDevices = 64;
 std::mutex g_pool_mu;
 cudaMemPool_t g_pools[kMaxDevices] = {};
@@ -87,7 +91,7 @@ bool capturing(cudaStream_t s) {
 void* device_alloc(size_t bytes, bool* pooled) {
     void* p = nullptr;
     cudaStream_t s = stream();
-    if (capturing(s)) {
+    if (bytes >= kPoolLargest || capturing(s)) {
         *pooled = false;
         RB_CUDA(cudaMalloc(&p, bytes));
         return p;
