@@ -353,7 +353,7 @@ int rb_spmv(rb_csr A, rb_vec x, rb_vec b) {
     return guarded([&]() -> int {
         NEED(A); NEED(x); NEED(b);
         RB_REQUIRE(x->n == A->n_cols && b->n == A->n_rows, "spmv: sizes do not match");
-        spmv64(view(*A), x->v.get(), b->v.get(), handle_lanes(*A, x->v.get()));
+        handle_spmv(*A, x->v.get(), b->v.get());
         return RB_OK;
     });
 }
@@ -363,7 +363,7 @@ int rb_residual(rb_csr A, rb_vec x, rb_vec b, rb_vec r) {
         NEED(A); NEED(x); NEED(b); NEED(r);
         RB_REQUIRE(x->n == A->n_cols && b->n == A->n_rows && r->n == A->n_rows,
                    "residual: sizes do not match");
-        residual64(view(*A), x->v.get(), b->v.get(), r->v.get(), handle_lanes(*A, x->v.get()));
+        handle_residual(*A, x->v.get(), b->v.get(), r->v.get());
         return RB_OK;
     });
 }
@@ -384,7 +384,7 @@ int rb_spmv_append(rb_csr A, rb_vec x, rb_vec b) {
     return guarded([&]() -> int {
         NEED(A); NEED(x); NEED(b);
         RB_REQUIRE(x->n == A->n_cols && b->n == A->n_rows, "spmv_append: sizes do not match");
-        spmv_append64(view(*A), x->v.get(), b->v.get(), handle_lanes(*A, x->v.get()));
+        handle_append(*A, x->v.get(), b->v.get());
         return RB_OK;
     });
 }

@@ -12,8 +12,16 @@ namespace rb {
 // order.  Built on the first transposed product and kept on the handle, so
 // later products gather A's current values through it (values may change
 // between calls, the pattern may not).
+//
+// The rows of a pattern with many entries, found once (the row lengths are
+// part of the pattern).
+struct LongRows {
+    DevArray<int> list;
+    int count = 0;
+};
 struct TransposeMap {
     DevArray<int> rowptr, rows, src;
+    LongRows longs;
 };
 }  // namespace rb
 
@@ -24,6 +32,7 @@ struct rb_csr_s {
     rb::DevArray<double> vals;
     std::unique_ptr<rb::TransposeMap> tmap;  // lazily built by spmv_T64
     int lanes = 0;  // row-kernel schedule of the public products (timed on first use)
+    rb::LongRows longs;
 };
 
 struct rb_batch_s;
@@ -92,13 +101,14 @@ void dot_async(const double* a, const double* b, int n, double* result_dev);
 
 // SpMV family on FP64 CSR (C ABI primitives); lanes 0 picks the row
 // schedule from the mean row length.
-void spmv64(const CsrView<double>& A, const double* x, double* y, int lanes = 0);
 void residual64(const CsrView<double>& A, const double* x, const double* b, double* r,
                 int lanes = 0);
-void spmv_append64(const CsrView<double>& A, const double* x, double* y, int lanes = 0);
 // The fastest row schedule for a handle's products, timed once on x (the
-// handle keeps it).
+// handle keeps it), and the products on it.
 int handle_lanes(rb_csr_s& A, const double* x);
+void handle_spmv(rb_csr_s& A, const double* x, double* y);
+void handle_residual(rb_csr_s& A, const double* x, const double* b, double* r);
+void handle_append(rb_csr_s& A, const double* x, double* y);
 // y = A^T x through the handle's cached transpose map (built on first use).
 void spmv_T64(rb_csr_s& A, const double* x, double* y);
 

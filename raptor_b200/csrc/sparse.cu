@@ -367,23 +367,130 @@ __global__ void k_to_int(long long nnz, const double* v, int* out) {
         out[k] = (int)v[k];
 }
 
-// y_j = sum over the entries of row j of A^T of vals[src] * x[row]: 8 lanes
-// per row, each lane a fixed stride of the row, then a fixed shuffle tree,
-// so the result does not depend on scheduling.
-__global__ void __launch_bounds__(256)
+// Rows (or columns, of a transpose map) with more than kLongRow entries: a
+// block of their own each, because on a few lanes their load chains outlast
+// the whole product (a column of 9000 entries on 8 lanes held a product of
+// 5.3M entries at 377 us).  256 entries are 8 batches of 4 on 8 lanes.
+constexpr int kLongRow = 256;
+constexpr int kRowsLong = 256;   // flag of a handle's lanes value
+
+__global__ void k_long_rows(int n, const int* __restrict__ rp, int* list, int* count) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && rp[i + 1] - rp[i] > kLongRow) list[atomicAdd(count, 1)] = i;
+}
+
+static void find_long_rows(int n, long long nnz, const int* rp, LongRows& L) {
+    L.count = 0;
+    if (n == 0 || nnz <= kLongRow) return;
+    L.list.alloc((size_t)std::min<long long>(n, nnz / kLongRow));
+    DevArray<int> count(1);
+    count.zero();
+    k_long_rows<<<grid_for(n, 256), 256, 0, stream()>>>(n, rp, L.list.get(), count.get());
+    RB_CHECK_LAUNCH();
+    L.count = read_scalar(count.get());
+    if (!L.count) L.list.release();
+}
+
+// Sum of t over a block of kRowBlock threads in a fixed order; thread 0 has it.
+__device__ __forceinline__ double block_sum(double t) {
+    __shared__ double part[kRowBlock / 32];
+    t = warp_sum(t);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = t;
+    __syncthreads();
+    double s = 0.0;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < kRowBlock / 32; w++) s += part[w];
+    return s;
+}
+
+// The strided row kernel with the long rows on blocks of their own (the
+// first nlong of the grid, so that they start at once).
+template <int G, class Epi>
+__global__ void __launch_bounds__(kRowBlock)
+k_csr_rows_long(long n, const int* __restrict__ rp, const int* __restrict__ ci,
+                const double* __restrict__ cv, const double* __restrict__ x, Epi epi,
+                const int* __restrict__ longs, int nlong) {
+    double red = 0.0;
+    if ((int)blockIdx.x < nlong) {
+        const int row = longs[blockIdx.x];
+        const double s = block_sum(row_batched<kRowBlock, RB_ROWS_BATCH, double>(
+            rp[row] + (int)threadIdx.x, rp[row + 1], ci, cv, x));
+        if (threadIdx.x == 0) epi((long)row, s, red);
+        return;
+    }
+    constexpr int RPW = 32 / G;
+    const int lane = threadIdx.x & 31;
+    const int sub = lane / G, gl = lane & (G - 1);
+    const long gwarp = ((long)(blockIdx.x - nlong) * blockDim.x + threadIdx.x) >> 5;
+    const long nwarps = ((long)(gridDim.x - nlong) * blockDim.x) >> 5;
+    for (long base = gwarp * RPW; base < n; base += nwarps * RPW) {
+        const long row = base + sub;
+        int s = 0, e = 0;
+        if (row < n) { s = __ldg(rp + row); e = __ldg(rp + row + 1); }
+        const bool mine = row < n && e - s <= kLongRow;
+        double sum = row_batched<G, RB_ROWS_BATCH, double>(s + gl, mine ? e : s, ci, cv, x);
+        sum = group_sum<G>(sum);
+        if (mine && gl == 0) epi(row, sum, red);
+    }
+}
+
+// y_j = sum over the entries of row j of A^T of vals[src] * x[row].  A
+// lane's share of a row is walked kTBatch entries at a time: the source
+// rows and positions of a batch, then its gathers of vals and x, then the
+// products in increasing position, so that the two dependent loads of a
+// batch overlap (one entry at a time on 8 lanes, a 27-point row took four
+// dependent round trips).  Fixed strides and a fixed shuffle tree: the
+// result does not depend on scheduling.
+constexpr int kTBatch = 4;
+template <int STEP>
+__device__ __forceinline__ double t_row(int k, int e, const int* __restrict__ rows,
+                                        const int* __restrict__ src,
+                                        const double* __restrict__ vals,
+                                        const double* __restrict__ x) {
+    double s = 0.0;
+    for (; k < e; k += kTBatch * STEP) {
+        int r[kTBatch], p[kTBatch];
+        double v[kTBatch], w[kTBatch];
+#pragma unroll
+        for (int q = 0; q < kTBatch; q++) {
+            const bool ok = k + q * STEP < e;
+            r[q] = ok ? __ldg(rows + k + q * STEP) : 0;
+            p[q] = ok ? __ldg(src + k + q * STEP) : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < kTBatch; q++) {
+            const bool ok = k + q * STEP < e;
+            v[q] = ok ? __ldg(vals + p[q]) : 0.0;
+            w[q] = ok ? __ldg(x + r[q]) : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < kTBatch; q++)
+            if (k + q * STEP < e) s += v[q] * w[q];
+    }
+    return s;
+}
+
+template <int G>
+__global__ void __launch_bounds__(kRowBlock)
 k_spmv_T_map(int n, const int* __restrict__ rp, const int* __restrict__ rows,
              const int* __restrict__ src, const double* __restrict__ vals,
-             const double* __restrict__ x, double* __restrict__ y) {
-    constexpr int G = 8;
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+             const double* __restrict__ x, double* __restrict__ y, const int* __restrict__ longs,
+             int nlong) {
+    if ((int)blockIdx.x < nlong) {
+        const int j = longs[blockIdx.x];
+        const double s = block_sum(t_row<kRowBlock>(rp[j] + (int)threadIdx.x, rp[j + 1], rows, src, vals, x));
+        if (threadIdx.x == 0) y[j] = s;
+        return;
+    }
+    const long t = (long)(blockIdx.x - nlong) * blockDim.x + threadIdx.x;
     const long j = t / G;
     const int g = threadIdx.x & (G - 1);
-    double s = 0.0;
-    if (j < n)
-        for (int k = rp[j] + g; k < rp[j + 1]; k += G) s += vals[src[k]] * x[rows[k]];
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, G);
-    if (j < n && g == 0) y[j] = s;
+    int b = 0, e = 0;
+    if (j < n) { b = __ldg(rp + j); e = __ldg(rp + j + 1); }
+    const bool mine = j < n && e - b <= kLongRow;
+    double s = t_row<G>(b + g, mine ? e : b, rows, src, vals, x);
+    s = group_sum<G>(s);
+    if (mine && g == 0) y[j] = s;
 }
 
 void spmv_T64(rb_csr_s& A, const double* x, double* y) {
@@ -404,13 +511,25 @@ void spmv_T64(rb_csr_s& A, const double* x, double* y) {
         RB_CHECK_LAUNCH();
         m->rowptr = std::move(T->rowptr);
         m->rows = std::move(T->cols);
+        find_long_rows(A.n_cols, A.nnz, m->rowptr.get(), m->longs);
         RB_CUDA(cudaStreamSynchronize(stream()));   // kept on the handle: complete on any stream
         A.tmap = std::move(m);
     }
-    if (A.n_cols)
-        k_spmv_T_map<<<grid_for((long)A.n_cols * 8, 256), 256, 0, stream()>>>(
-            A.n_cols, A.tmap->rowptr.get(), A.tmap->rows.get(), A.tmap->src.get(), A.vals.get(),
-            x, y);
+    if (!A.n_cols) return;
+    const TransposeMap& m = *A.tmap;
+    auto launch = [&](auto g) {
+        constexpr int G = decltype(g)::value;
+        k_spmv_T_map<G><<<grid_for((long)A.n_cols * G, kRowBlock) + m.longs.count, kRowBlock, 0, stream()>>>(
+            A.n_cols, m.rowptr.get(), m.rows.get(), m.src.get(), A.vals.get(), x, y,
+            m.longs.list.get(), m.longs.count);
+    };
+    // Lanes a row from the mean length.  Measured with 2 / 4 / 8 / 16 lanes
+    // (us): 27 entries a row (128^3) 226 / 182 / 199 / 317, 18 (300k ragged
+    // rows) 44 / 43 / 46 / 58, 9 (1000^2) 45 / 47 / 73 / 128, 5 within noise;
+    // 8 lanes and one entry at a time took 209 us on the first, and 377 us
+    // on the second, whose longest row has 9000 entries.
+    if ((double)A.nnz > 12.0 * A.n_cols) launch(std::integral_constant<int, 4>{});
+    else launch(std::integral_constant<int, 2>{});
     RB_CHECK_LAUNCH();
 }
 
@@ -466,18 +585,43 @@ void dot_async(const double* a, const double* b, int n, double* result_dev) {
 }
 
 // ------------------------------------------------------- FP64 SpMV ops --
-void spmv64(const CsrView<double>& A, const double* x, double* y, int lanes) {
-    launch_rows(A.rowptr, A.cols, A.vals, A.n_rows, A.nnz, x, EpiStore<double>{y}, lanes);
-}
-
 void residual64(const CsrView<double>& A, const double* x, const double* b, double* r,
                 int lanes) {
     launch_rows(A.rowptr, A.cols, A.vals, A.n_rows, A.nnz, x, EpiResidual<double, double>{b, r},
                 lanes);
 }
 
-void spmv_append64(const CsrView<double>& A, const double* x, double* y, int lanes) {
-    launch_rows(A.rowptr, A.cols, A.vals, A.n_rows, A.nnz, x, EpiAppend<double>{y}, lanes);
+// A handle's products: on the schedule picked for it, with its long rows on
+// blocks of their own when that was the fastest (kRowsLong).
+template <class Epi>
+static void handle_rows(rb_csr_s& A, const double* x, Epi epi, int lanes) {
+    if (!(lanes & kRowsLong)) {
+        launch_rows(A.rowptr.get(), A.cols.get(), A.vals.get(), A.n_rows, A.nnz, x, epi, lanes);
+        return;
+    }
+    const int nl = A.longs.count;
+    auto launch = [&](auto g) {
+        constexpr int G = decltype(g)::value;
+        k_csr_rows_long<G><<<row_grid(A.n_rows, G) + nl, kRowBlock, 0, stream()>>>(
+            A.n_rows, A.rowptr.get(), A.cols.get(), A.vals.get(), x, epi, A.longs.list.get(), nl);
+    };
+    switch (lanes & (kRowsBlocked - 1)) {
+        case 2: launch(std::integral_constant<int, 2>{}); break;
+        case 4: launch(std::integral_constant<int, 4>{}); break;
+        case 8: launch(std::integral_constant<int, 8>{}); break;
+        default: launch(std::integral_constant<int, 16>{}); break;
+    }
+    RB_CHECK_LAUNCH();
+}
+
+void handle_spmv(rb_csr_s& A, const double* x, double* y) {
+    handle_rows(A, x, EpiStore<double>{y}, handle_lanes(A, x));
+}
+void handle_residual(rb_csr_s& A, const double* x, const double* b, double* r) {
+    handle_rows(A, x, EpiResidual<double, double>{b, r}, handle_lanes(A, x));
+}
+void handle_append(rb_csr_s& A, const double* x, double* y) {
+    handle_rows(A, x, EpiAppend<double>{y}, handle_lanes(A, x));
 }
 
 int handle_lanes(rb_csr_s& A, const double* x) {
@@ -493,11 +637,15 @@ int handle_lanes(rb_csr_s& A, const double* x) {
     RB_CUDA(cudaEventCreate(&e1));
     float best = 1e30f;
     int bestG = pick_group(A.n_rows, A.nnz);
-    const CsrView<double> v = view(A);
-    for (int G : cands) {
-        spmv64(v, x, y.get(), G);
+    std::vector<int> tries(cands, cands + 10);
+    find_long_rows(A.n_rows, A.nnz, A.rowptr.get(), A.longs);
+    if (A.longs.count)
+        for (int G : {2, 4, 8, 16}) tries.push_back(kRowsLong | G);
+    const EpiStore<double> out{y.get()};
+    for (int G : tries) {
+        handle_rows(A, x, out, G);
         RB_CUDA(cudaEventRecord(e0, stream()));
-        for (int rep = 0; rep < 3; rep++) spmv64(v, x, y.get(), G);
+        for (int rep = 0; rep < 3; rep++) handle_rows(A, x, out, G);
         RB_CUDA(cudaEventRecord(e1, stream()));
         RB_CUDA(cudaEventSynchronize(e1));
         float ms = 0;
