@@ -140,11 +140,20 @@ void apply_A_block(const Level<T>& V, const BLevel<T>& W, const T* X, int k, Epi
     else launch_csr_block(V.A.rowptr, V.A.cols, V.A.vals, V.n, k, X, epi, W.sA);
 }
 
-// Tile shape of one SpMM: rows split S in {1, 2, 4} (S KP <= 32), timed.
+// Tile shape of one SpMM: rows split S, timed; S in {1, 2, 4} (S KP <= 32),
+// or up to 8 where the 16-byte column groups apply (vec_split).  Operators
+// too small to time take a split that leaves a lane about 8 entries.
 template <typename T>
 int tune_split(const CsrView<T>& M, int k, const T* xin, T* yout, const char* op) {
     const int KP = pow2_at_least(k);
-    if (M.n_rows < 4096 || KP >= 32) return 1;
+    const int lpr = vec_lanes(k, xin, BStore<T>{yout});
+    if (M.n_rows < 4096) {
+        if (!lpr || M.n_rows == 0) return 1;
+        int S = 1;
+        while (S < 8 && (double)M.nnz > 8.0 * S * M.n_rows) S *= 2;
+        return vec_split(lpr, S);
+    }
+    if (!lpr && KP >= 32) return 1;
     const std::string key = tune_key((std::string(op) + std::to_string(k)).c_str(), M.n_rows,
                                      M.nnz, (int)sizeof(T));
     auto& c = tune_cache();
@@ -152,7 +161,7 @@ int tune_split(const CsrView<T>& M, int k, const T* xin, T* yout, const char* op
     if (it != c.m.end()) return it->second;
     float best = 1e30f;
     int bestS = 1;
-    for (int S = 1; S <= 4 && S * KP <= 32; S <<= 1) {
+    for (int S = 1; lpr ? vec_split(lpr, S) == S : (S <= 4 && S * KP <= 32); S <<= 1) {
         const float t = time_launch([&] {
             launch_csr_block(M.rowptr, M.cols, M.vals, M.n_rows, k, xin, BStore<T>{yout}, S);
         }, xin, sizeof(T) * (size_t)M.n_cols * (size_t)k);

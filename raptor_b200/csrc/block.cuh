@@ -436,37 +436,39 @@ k_csr_block_dot(long n, int k, const int* __restrict__ rp, const int* __restrict
 }
 
 // ------------------------------------------------ vectorised CSR SpMM --
-// LPR = KP / VW lanes a row, each with VW columns (Vec16); 32 / LPR rows a
-// warp step.  The row's indices and values are broadcast loads (the LPR
-// lanes of a row read the same entry); every lane then has the 16-byte
-// gathers of up to RB_BLOCK_VEC_UN nonzeros in flight before it uses the
-// first.  Each column's products are added in increasing position, as in
-// k_csr_block with one row split.
+// LPR = KP / VW lanes cover a row's columns, VW each (Vec16), and S such
+// groups split the row's nonzeros: group s takes entries s, s + S, ... and a
+// shuffle tree adds the groups, 32 / (LPR S) rows a warp step.  The LPR lanes
+// of a group read the same index and value, neighbouring groups neighbouring
+// ones; every lane then has the 16-byte gathers of up to UN nonzeros in
+// flight before it uses the first.  One group a row (S = 1) left a coarse
+// operator's rows (50 to 130 entries, few rows) on two lanes each: a serial
+// chain of up to 16 batches and most of the chip idle.
 #ifndef RB_BLOCK_VEC_UN
 #define RB_BLOCK_VEC_UN 8
 #endif
 
-template <int LPR, typename TV, typename TX, typename Acc>
+template <int LPR, int S, typename TV, typename TX, typename Acc>
 __device__ __forceinline__ void csr_row_v(int rs, int re, bool on, const int* __restrict__ ci,
                                           const TV* __restrict__ cv, const TX* __restrict__ X,
                                           int k, int c0, Acc (&acc)[Vec16<TX>::n]) {
     constexpr int VW = Vec16<TX>::n;
-    constexpr int UN = RB_BLOCK_VEC_UN;
+    constexpr int UN = S == 1 ? RB_BLOCK_VEC_UN : RB_BLOCK_VEC_UN / 2;
 #pragma unroll
     for (int v = 0; v < VW; v++) acc[v] = Acc(0);
-    for (int j = rs; j < re; j += UN) {
+    for (int j = rs; j < re; j += UN * S) {
         int cc[UN];
         TV vv[UN];
 #pragma unroll
         for (int u = 0; u < UN; u++) {
-            const bool in = j + u < re;
-            cc[u] = in ? __ldg(ci + j + u) : 0;
-            vv[u] = in ? __ldg(cv + j + u) : TV(0);
+            const bool in = j + u * S < re;
+            cc[u] = in ? __ldg(ci + j + u * S) : 0;
+            vv[u] = in ? __ldg(cv + j + u * S) : TV(0);
         }
         TX xx[UN][VW];
 #pragma unroll
         for (int u = 0; u < UN; u++) {
-            if (on && j + u < re) {
+            if (on && j + u * S < re) {
                 vload_ro<TX, VW>(X + (long)cc[u] * k + c0, xx[u]);
             } else {
 #pragma unroll
@@ -475,20 +477,24 @@ __device__ __forceinline__ void csr_row_v(int rs, int re, bool on, const int* __
         }
 #pragma unroll
         for (int u = 0; u < UN; u++)
-            if (j + u < re)
+            if (j + u * S < re)
 #pragma unroll
                 for (int v = 0; v < VW; v++) acc[v] += (Acc)vv[u] * (Acc)xx[u][v];
     }
+#pragma unroll
+    for (int o = LPR; o < LPR * S; o <<= 1)
+#pragma unroll
+        for (int v = 0; v < VW; v++) acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], o);
 }
 
-template <int LPR, typename TV, typename TX, typename Acc, class Epi>
+template <int LPR, int S, typename TV, typename TX, typename Acc, class Epi>
 __global__ void __launch_bounds__(256)
 k_csr_block_v(long n, int k, const int* __restrict__ rp, const int* __restrict__ ci,
               const TV* __restrict__ cv, const TX* __restrict__ X, Epi epi) {
     constexpr int VW = Vec16<TX>::n;
-    constexpr int RPW = 32 / LPR;
+    constexpr int RPW = 32 / (LPR * S);
     const int lane = threadIdx.x & 31;
-    const int c0 = (lane % LPR) * VW, sub = lane / LPR;
+    const int c0 = (lane % LPR) * VW, s = (lane / LPR) % S, sub = lane / (LPR * S);
     const long gwarp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
     for (long base = gwarp * RPW; base < n; base += nwarps * RPW) {
@@ -497,21 +503,21 @@ k_csr_block_v(long n, int k, const int* __restrict__ rp, const int* __restrict__
         int rs = 0, re = 0;
         if (row < n) { rs = __ldg(rp + row); re = __ldg(rp + row + 1); }
         Acc acc[VW];
-        csr_row_v<LPR, TV, TX, Acc>(rs, re, on, ci, cv, X, k, c0, acc);
-        if (on) epi.template vec<VW>(row, c0, k, acc);
+        csr_row_v<LPR, S, TV, TX, Acc>(rs + s, re, on, ci, cv, X, k, c0, acc);
+        if (on && s == 0) epi.template vec<VW>(row, c0, k, acc);
     }
 }
 
 // Y = A P with the per-column dots p.y, VW columns a lane
-template <int LPR, typename TV, class Fin>
+template <int LPR, int S, typename TV, class Fin>
 __global__ void __launch_bounds__(256)
 k_csr_block_dot_v(long n, int k, const int* __restrict__ rp, const int* __restrict__ ci,
                   const TV* __restrict__ cv, const double* __restrict__ P, double* __restrict__ Y,
                   ReduceSlot rsl, Fin fin) {
     constexpr int VW = Vec16<double>::n;
-    constexpr int RPW = 32 / LPR;
+    constexpr int RPW = 32 / (LPR * S);
     const int lane = threadIdx.x & 31;
-    const int c0 = (lane % LPR) * VW, sub = lane / LPR;
+    const int c0 = (lane % LPR) * VW, s = (lane / LPR) % S, sub = lane / (LPR * S);
     const long gwarp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
     double red[VW];
@@ -523,8 +529,8 @@ k_csr_block_dot_v(long n, int k, const int* __restrict__ rp, const int* __restri
         int rs = 0, re = 0;
         if (row < n) { rs = __ldg(rp + row); re = __ldg(rp + row + 1); }
         double acc[VW];
-        csr_row_v<LPR, TV, double, double>(rs, re, on, ci, cv, P, k, c0, acc);
-        if (on) {
+        csr_row_v<LPR, S, TV, double, double>(rs + s, re, on, ci, cv, P, k, c0, acc);
+        if (on && s == 0) {
             double pp[VW];
             vload_ro<double, VW>(P + row * k + c0, pp);
             vstore<double, VW>(Y + row * k + c0, acc);
@@ -889,6 +895,23 @@ int vec_lanes(int k, const TX* X, const Epi& epi) {
         default: { constexpr int kL = 16; __VA_ARGS__; } break;    \
     }
 
+// Row splits S of the vectorised CSR kernels: 1, 2, 4 or 8 groups of LPR
+// lanes, at most kVecSplitLanes lanes a row (a wider row group would idle on
+// the epilogue's columns).
+constexpr int kVecSplitLanes = 16;
+inline int vec_split(int lpr, int S) {
+    int s = 1;
+    while (s < 8 && 2 * s <= S && 2 * s * lpr <= kVecSplitLanes) s *= 2;
+    return s;
+}
+template <int L, class F>
+void vec_split_switch(int s, F&& f) {
+    if constexpr (L * 8 <= kVecSplitLanes) if (s == 8) { f(std::integral_constant<int, 8>{}); return; }
+    if constexpr (L * 4 <= kVecSplitLanes) if (s == 4) { f(std::integral_constant<int, 4>{}); return; }
+    if constexpr (L * 2 <= kVecSplitLanes) if (s == 2) { f(std::integral_constant<int, 2>{}); return; }
+    f(std::integral_constant<int, 1>{});
+}
+
 template <typename TV, typename TX, class Epi>
 void launch_csr_block(const int* rp, const int* ci, const TV* cv, long n, int k, const TX* X,
                       Epi epi, int S) {
@@ -896,9 +919,12 @@ void launch_csr_block(const int* rp, const int* ci, const TV* cv, long n, int k,
     using Acc = AccOf2<TV, TX>;
     if (const int lpr = vec_lanes(k, X, epi)) {
         RB_BLOCK_LPR_SWITCH(lpr, {
-            auto kern = k_csr_block_v<kL, TV, TX, Acc, Epi>;
-            const unsigned g = block_grid_gather((const void*)kern, n, kL, 1);
-            kern<<<g, 256, 0, stream()>>>(n, k, rp, ci, cv, X, epi);
+            vec_split_switch<kL>(vec_split(lpr, S), [&](auto sp) {
+                constexpr int kS = decltype(sp)::value;
+                auto kern = k_csr_block_v<kL, kS, TV, TX, Acc, Epi>;
+                const unsigned g = block_grid_gather((const void*)kern, n, kL, kS);
+                kern<<<g, 256, 0, stream()>>>(n, k, rp, ci, cv, X, epi);
+            });
         });
         RB_CHECK_LAUNCH();
         return;
@@ -929,10 +955,13 @@ void launch_csr_block_dot(const int* rp, const int* ci, const TV* cv, long n, in
                           const double* P, double* Y, int S, Fin fin) {
     if (const int lpr = vec_lanes(k, P, BStore<double>{Y})) {
         RB_BLOCK_LPR_SWITCH(lpr, {
-            auto kern = k_csr_block_dot_v<kL, TV, Fin>;
-            const unsigned g = block_grid_gather((const void*)kern, n, kL, 1);
-            ReduceSlot rs = global_reduce_slot((int)g * kMaxBlockK);
-            kern<<<g, 256, 0, stream()>>>(n, k, rp, ci, cv, P, Y, rs, fin);
+            vec_split_switch<kL>(vec_split(lpr, S), [&](auto sp) {
+                constexpr int kS = decltype(sp)::value;
+                auto kern = k_csr_block_dot_v<kL, kS, TV, Fin>;
+                const unsigned g = block_grid_gather((const void*)kern, n, kL, kS);
+                ReduceSlot rs = global_reduce_slot((int)g * kMaxBlockK);
+                kern<<<g, 256, 0, stream()>>>(n, k, rp, ci, cv, P, Y, rs, fin);
+            });
         });
         RB_CHECK_LAUNCH();
         return;

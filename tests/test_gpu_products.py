@@ -55,3 +55,30 @@ def test_products_with_long_rows_and_columns(n, m, mean, special):
     assert np.all(np.abs(r.numpy() - (uh - want)) <= 2 * bound)
     assert np.all(np.abs(a.numpy() - (uh + want)) <= 2 * bound)
     assert np.all(np.abs(t.numpy() - wantT) <= eps * (np.bincount(cols, minlength=m) + 2) * scaleT + 1e-300)
+
+
+@pytest.mark.parametrize("prec", [rb.FP64, rb.FP32], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("k", [4, 8, 12, 16, 24])
+def test_block_cycle_with_split_rows(prec, k):
+    """Column groups of 16 bytes with a row's entries split over 1 to 8
+    groups: levels above and below the size whose split is timed, against one
+    single-vector cycle a column (the order of the sums is all that
+    differs)."""
+    m = 26
+    st = [0.0] * 27
+    st[13], st[12], st[14], st[10], st[16], st[4], st[22] = 4.02, -1, -1, -1, -1, -0.01, -0.01
+    A = rb.par_stencil_grid(st, [m, m, m])
+    n = A.global_num_rows
+    ml = rb.ParSmoothedAggregationSolver(0.25, relax_type=rb.L1Jacobi)
+    ml.precision = prec
+    ml.setup(A)
+    Bh = np.random.default_rng(k).uniform(-1, 1, (n, k))
+    X = rb.ParVector(n * k)
+    ml.cycle_block(X, rb.ParVector(n * k, values=Bh.reshape(-1)), k)
+    got = X.numpy().reshape(n, k)
+    tol = 1e-11 if prec == rb.FP64 else 1e-5
+    for c in range(k):
+        x = rb.ParVector(n)
+        ml.cycle(x, rb.ParVector(n, values=Bh[:, c]))
+        ref = x.numpy()
+        assert np.linalg.norm(got[:, c] - ref) <= tol * np.linalg.norm(ref), c
