@@ -252,6 +252,7 @@ int adjoint_solve(const rb_csr_s& A, Hierarchy& H, double* lambda, const double*
                                             sizeof(double) * T->lv64[l].n, cudaMemcpyDeviceToDevice,
                                             stream()));
             }
+            T->build_bottom();   // of the replaced diagonals
             H.adj_AT.reset(transpose(A));
             T->src_A = H.adj_AT.get();
             H.adj = std::move(T);

@@ -1,0 +1,150 @@
+// dense_bottom.cuh -- the bottom of the V-cycle as one dense product.
+//
+// From a zero guess, the part of the cycle from level f down is linear in its
+// right-hand side: x_f = B b_f with a fixed n_f x n_f matrix B.  Level by
+// level it costs five small kernels a level (2 us of launch and drain each,
+// 4 to 17 us for the coarsest solve or the cluster tail), whatever their
+// size; B of a level of a thousand rows is 4 MB in FP32, which the L2 holds,
+// and one product with it takes about 3 us.  Setup forms B once, in FP64 from
+// the FP64 hierarchy, upwards from the inverse of the coarsest matrix:
+//
+//     T = R (I - A D)         restriction of the first sweep's residual
+//     E = B_c T               the level below
+//     X = D + P E             first sweep plus coarse correction
+//     B = X + D (I - A X)     post-sweep
+//
+// with D the smoother's scaled inverse diagonal (no sweeps: B = P B_c R),
+// and rounds it once to the cycle's precision.  The product accumulates in
+// FP64.
+#pragma once
+
+#include "rb_common.cuh"
+
+namespace rb {
+
+// Bytes of the largest B: 16 MB, of which the L2 (126 MB) keeps what a
+// cycle's other levels leave; a product at that size reads about as long as
+// two of the launches it replaces take.
+constexpr size_t kDenseBytes = (size_t)16 << 20;
+
+// Row length of B in elements of T: rows start on 16-byte boundaries.
+template <typename T>
+inline int dense_ld(int n) {
+    constexpr int v = 16 / sizeof(T);
+    return (n + v - 1) / v * v;
+}
+
+// x = B b: one warp a row, 16 bytes a lane and step.  Rows are padded with
+// zeros to ld, and b is read only below n.
+template <typename T>
+__global__ void __launch_bounds__(128)
+k_dense_mv(int n, int ld, const T* __restrict__ B, const T* __restrict__ b, T* __restrict__ x) {
+    constexpr int V = 16 / sizeof(T);
+    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (row >= n) return;
+    const T* r = B + (size_t)row * ld;
+    double s = 0.0;
+#pragma unroll 4
+    for (int j = lane * V; j < ld; j += 32 * V) {
+        T a[V];
+        *reinterpret_cast<uint4*>(a) = __ldg(reinterpret_cast<const uint4*>(r + j));
+#pragma unroll
+        for (int v = 0; v < V; v++) s += (double)a[v] * (j + v < n ? (double)__ldg(b + j + v) : 0.0);
+    }
+    s = warp_sum(s);
+    if (lane == 0) x[row] = (T)s;
+}
+
+// ------------------------------------------------------- forming B (FP64) --
+// out (n x m, row-major) = the transpose of a column-major n x n matrix
+static __global__ void k_dense_from_inverse(int n, const double* __restrict__ inv, double* out) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
+    if (c < n) out[(size_t)i * n + c] = inv[(size_t)c * n + i];
+}
+
+// M = I - A D, one thread a row (M zeroed before)
+template <typename T>
+__global__ void k_dense_first_residual(int n, const int* __restrict__ rp, const int* __restrict__ ci,
+                                       const double* __restrict__ cv, const T* __restrict__ d,
+                                       double* M) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double* row = M + (size_t)i * n;
+    row[i] = 1.0;
+    for (int j = rp[i]; j < rp[i + 1]; j++) row[ci[j]] -= cv[j] * (double)d[ci[j]];
+}
+
+// M = the CSR matrix, dense with m columns (M zeroed before)
+static __global__ void k_dense_copy(int n, int m, const int* __restrict__ rp,
+                                    const int* __restrict__ ci, const double* __restrict__ cv,
+                                    double* M) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    for (int j = rp[i]; j < rp[i + 1]; j++) M[(size_t)i * m + ci[j]] += cv[j];
+}
+
+// Y = S X for CSR S (rows of Y one a blockIdx.y, m columns), then
+// MODE 0: out = Y;  1: out = diag(d) + Y;  2: out = X + diag(d) (I - Y),
+// S square.
+template <int MODE, typename T>
+__global__ void __launch_bounds__(256)
+k_dense_spmm(int m, const int* __restrict__ rp, const int* __restrict__ ci,
+             const double* __restrict__ cv, const double* __restrict__ X, const T* __restrict__ d,
+             double* __restrict__ out) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
+    if (c >= m) return;
+    double s = 0.0;
+    const int e = rp[i + 1];
+#pragma unroll 4
+    for (int j = rp[i]; j < e; j++) s += cv[j] * X[(size_t)ci[j] * m + c];
+    if (MODE == 1) s += c == i ? (double)d[i] : 0.0;
+    if (MODE == 2) s = X[(size_t)i * m + c] + (double)d[i] * ((c == i ? 1.0 : 0.0) - s);
+    out[(size_t)i * m + c] = s;
+}
+
+// C (n x m) = A (n x n) B (n x m), FP64, row-major: 32 x 64 tiles, 256
+// threads of 2 x 4 entries, 16 of the inner dimension a step.
+static __global__ void __launch_bounds__(256)
+k_dense_gemm(int n, int m, const double* __restrict__ A, const double* __restrict__ B,
+             double* __restrict__ C) {
+    __shared__ double sa[16][33], sb[16][64];
+    const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 64;
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    double acc[2][4] = {};
+    for (int k0 = 0; k0 < n; k0 += 16) {
+        for (int t = threadIdx.x; t < 32 * 16; t += 256) {
+            const int r = t / 16, k = t % 16;
+            sa[k][r] = r0 + r < n && k0 + k < n ? A[(size_t)(r0 + r) * n + k0 + k] : 0.0;
+        }
+        for (int t = threadIdx.x; t < 16 * 64; t += 256) {
+            const int k = t / 64, c = t % 64;
+            sb[k][c] = k0 + k < n && c0 + c < m ? B[(size_t)(k0 + k) * m + c0 + c] : 0.0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            const double a0 = sa[k][ty * 2], a1 = sa[k][ty * 2 + 1];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const double b = sb[k][tx + 16 * q];
+                acc[0][q] += a0 * b;
+                acc[1][q] += a1 * b;
+            }
+        }
+        __syncthreads();
+    }
+    for (int p = 0; p < 2; p++)
+        for (int q = 0; q < 4; q++) {
+            const int r = r0 + ty * 2 + p, c = c0 + tx + 16 * q;
+            if (r < n && c < m) C[(size_t)r * m + c] = acc[p][q];
+        }
+}
+
+// B in the cycle precision, rows padded to ld
+template <typename T>
+__global__ void k_dense_store(int n, int ld, const double* __restrict__ in, T* __restrict__ out) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
+    if (c < ld) out[(size_t)i * ld + c] = c < n ? (T)in[(size_t)i * n + c] : T(0);
+}
+
+}  // namespace rb

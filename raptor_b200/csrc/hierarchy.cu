@@ -14,8 +14,10 @@
 #include <cmath>
 #include <map>
 #include <memory>
+#include <tuple>
 
 #include "blas1.cuh"
+#include "dense_bottom.cuh"
 #include "hierarchy.cuh"
 
 namespace rb {
@@ -940,8 +942,87 @@ void Hierarchy::build_cycle_data() {
     if (!host_scal) host_scal = static_cast<KScal*>(pinned_block());
     if (!host_ctl) host_ctl = static_cast<PcgCtl*>(pinned_block());
     gA0 = autotune_group(view(*master[0].A), kp.get(), kAp.get(), "A0_fp64");
-    if (opts.precision == RB_PREC_FP32) tune_tail(lv32, tdesc32);
-    else tune_tail(lv64, tdesc64);
+    build_bottom();
+}
+
+void Hierarchy::build_bottom() {
+    release_graphs();
+    if (opts.precision == RB_PREC_FP32) build_dense(lv32, dense32);
+    else build_dense(lv64, dense64);
+    if (dense_from >= 0) {
+        tail_from = -1;
+        tail_ms.clear();
+    } else if (opts.precision == RB_PREC_FP32) {
+        tune_tail(lv32, tdesc32);
+    } else {
+        tune_tail(lv64, tdesc64);
+    }
+}
+
+// The dense bottom starts at the first level f >= 1, above the coarsest,
+// whose matrix B fits kDenseBytes; it needs what the cluster tail needs (one
+// Jacobi-type sweep or the reference's no-op Jacobi, the explicit coarse
+// inverse) and is the default (fuse_coarse = 1; a forced tail start or 0
+// leaves it off).  Always taken where it applies: it replaces at least six
+// launches by one.
+template <typename T>
+void Hierarchy::build_dense(std::vector<Level<T>>& lv, DevArray<T>& B) {
+    dense_from = -1;
+    B.release();
+    const int L = (int)lv.size();
+    const int rt = opts.relax_type;
+    const bool none = rt == RB_RELAX_JACOBI && opts.jacobi_compat;
+    const bool jac = (rt == RB_RELAX_JACOBI || rt == RB_RELAX_L1JACOBI) &&
+                     (opts.num_smooth_sweeps == 1 || none);
+    if (opts.fuse_coarse != 1 || !jac || L < 3 || !cinv.get()) return;
+    int f = -1;
+    for (int l = L - 2; l >= 1; l--) {
+        const size_t n = (size_t)lv[l].n;
+        if (n == 0 || n * (size_t)dense_ld<T>(lv[l].n) * sizeof(T) > kDenseBytes) break;
+        f = l;
+    }
+    if (f < 0) return;
+    auto cols = [](int m) { return (unsigned)((m + 255) / 256); };
+    auto sp = [](const rb_csr_s& M) { return std::make_tuple(M.rowptr.get(), M.cols.get(), M.vals.get()); };
+    DevArray<double> Bc((size_t)coarse_n * coarse_n);
+    k_dense_from_inverse<<<dim3(cols(coarse_n), coarse_n), 256, 0, stream()>>>(coarse_n, cinv.get(), Bc.get());
+    RB_CHECK_LAUNCH();
+    for (int l = L - 2; l >= f; l--) {
+        const int n = lv[l].n, nc = lv[l + 1].n;
+        const T* d = lv[l].dinv.get();
+        const auto [arp, aci, acv] = sp(*master[l].A);
+        const auto [prp, pci, pcv] = sp(*master[l].P);
+        const auto [rrp, rci, rcv] = sp(*master[l].R);
+        const size_t nn = (size_t)n * n, cn = (size_t)nc * n;
+        DevArray<double> W(nn), Tm(cn), E(cn), Bl(nn);
+        if (none) {
+            Tm.zero();
+            k_dense_copy<<<grid_for(nc, 128), 128, 0, stream()>>>(nc, n, rrp, rci, rcv, Tm.get());
+        } else {
+            W.zero();
+            k_dense_first_residual<T><<<grid_for(n, 128), 128, 0, stream()>>>(n, arp, aci, acv, d, W.get());
+            RB_CHECK_LAUNCH();
+            k_dense_spmm<0, T><<<dim3(cols(n), nc), 256, 0, stream()>>>(n, rrp, rci, rcv, W.get(), d, Tm.get());
+        }
+        RB_CHECK_LAUNCH();
+        k_dense_gemm<<<dim3((n + 63) / 64, (nc + 31) / 32), 256, 0, stream()>>>(nc, n, Bc.get(), Tm.get(), E.get());
+        RB_CHECK_LAUNCH();
+        if (none) {
+            k_dense_spmm<0, T><<<dim3(cols(n), n), 256, 0, stream()>>>(n, prp, pci, pcv, E.get(), d, Bl.get());
+        } else {
+            k_dense_spmm<1, T><<<dim3(cols(n), n), 256, 0, stream()>>>(n, prp, pci, pcv, E.get(), d, W.get());
+            RB_CHECK_LAUNCH();
+            k_dense_spmm<2, T><<<dim3(cols(n), n), 256, 0, stream()>>>(n, arp, aci, acv, W.get(), d, Bl.get());
+        }
+        RB_CHECK_LAUNCH();
+        Bc = std::move(Bl);
+    }
+    const int n = lv[f].n;
+    dense_ld_ = dense_ld<T>(n);
+    B.alloc((size_t)n * dense_ld_);
+    k_dense_store<T><<<dim3(cols(dense_ld_), n), 256, 0, stream()>>>(n, dense_ld_, Bc.get(), B.get());
+    RB_CHECK_LAUNCH();
+    dense_from = f;
 }
 
 Hierarchy::~Hierarchy() {
@@ -1169,6 +1250,18 @@ void Hierarchy::cycle_level(std::vector<Level<T>>& lv, int l, T* x, const T* b, 
         else if (coarse_n)
             k_lu_solve<T><<<1, 256, sizeof(double) * coarse_n, stream()>>>(coarse_n, lu.get(),
                                                                           piv.get(), b, x);
+        RB_CHECK_LAUNCH();
+        mark(l * kProfSlots + 5);
+        return;
+    }
+    if (l == dense_from) {
+        // (from a zero guess, as every level below the finest starts; the
+        // profile books it as level dense_from's slot 5)
+        const T* B;
+        if constexpr (std::is_same<T, float>::value) B = dense32.get();
+        else B = dense64.get();
+        mark(l * kProfSlots + 6);
+        k_dense_mv<T><<<(V.n + 3) / 4, 128, 0, stream()>>>(V.n, dense_ld_, B, b, x);
         RB_CHECK_LAUNCH();
         mark(l * kProfSlots + 5);
         return;

@@ -168,6 +168,15 @@ struct Hierarchy {
     template <typename T>
     void tune_tail(std::vector<Level<T>>& lv, DevArray<LevelDesc<T>>& desc);
     std::vector<double> tail_ms;   // cycle ms per candidate start (tuning record)
+    // bottom of the cycle (levels dense_from .. L-1) as one dense product
+    // (dense_bottom.cuh); dense_from = -1: off
+    int dense_from = -1;
+    int dense_ld_ = 0;
+    DevArray<double> dense64;
+    DevArray<float> dense32;
+    template <typename T>
+    void build_dense(std::vector<Level<T>>& lv, DevArray<T>& B);
+    void build_bottom();   // the dense product where it applies, else the timed tail
     std::map<std::string, cudaGraphExec_t> graphs;
     std::map<std::string, long long> graph_kernels;
     // the matrix handed to setup: PCG on it reads the hierarchy's copies of
