@@ -26,7 +26,11 @@ namespace rb {
 
 namespace {
 
-constexpr int kSegChunk = 16384;   // rows per reduction chunk (chunks never span systems)
+// Rows per reduction chunk, one block each (chunks never span systems): 2048
+// rows are 8 loads of each operand a thread.  Of 16384 rows, a batch of 0.4
+// million had 30 blocks and a dot took 34 us (with a second kernel of 4 us
+// for the sums); this way 9 us.
+constexpr int kSegChunk = 2048;
 
 struct SegScal {
     double* rz;
@@ -115,43 +119,58 @@ __global__ void k_coarse_mv_batch(const int* __restrict__ row0, const int* __res
     }
 }
 
-// Segmented dot: one CTA per chunk writes its partial; then one thread per
-// system sums that system's chunks in order.  Deterministic.
+// Segmented dot: one CTA per chunk writes its partial, and the last CTA to
+// finish sums every system's partials, a warp a system: lanes take the
+// system's chunks in a fixed stride and meet in a fixed shuffle tree.
+// Deterministic.
 // gate (optional): the pass runs only when *gate is nonzero (a step of the
 // device-side loop that some iterations skip)
 // csys / active (optional): a chunk of a stopped system writes 0 unread.
+template <class Fin>
 __global__ void __launch_bounds__(256)
-k_seg_partial(const int* __restrict__ lo, const int* __restrict__ hi, const double* __restrict__ a,
-              const double* __restrict__ b, double* part, const int* gate,
-              const int* __restrict__ csys, const int* __restrict__ active) {
+k_seg_dot(const int* __restrict__ lo, const int* __restrict__ hi, const double* __restrict__ a,
+          const double* __restrict__ b, double* part, const int* gate,
+          const int* __restrict__ csys, const int* __restrict__ active, int n_sys,
+          const int* __restrict__ chunk0, unsigned* ticket, Fin fin) {
     if (gate && *(volatile const int*)gate == 0) return;
     __shared__ double w[8];
+    __shared__ bool is_last;
     const int c = blockIdx.x;
-    if (active && !active[csys[c]]) {
-        if (threadIdx.x == 0) part[c] = 0.0;
-        return;
-    }
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     double t = 0.0;
-    for (int i = lo[c] + threadIdx.x; i < hi[c]; i += blockDim.x) t += a[i] * b[i];
+    if (!active || active[csys[c]]) {
+        const int e = hi[c];
+        int i = lo[c] + threadIdx.x;
+        for (; i + 3 * 256 < e; i += 4 * 256) {
+            double u[4], v[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) { u[q] = a[i + q * 256]; v[q] = b[i + q * 256]; }
+#pragma unroll
+            for (int q = 0; q < 4; q++) t += u[q] * v[q];
+        }
+        for (; i < e; i += 256) t += a[i] * b[i];
+    }
     t = warp_sum(t);
-    if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = t;
+    if (lane == 0) w[wid] = t;
     __syncthreads();
     if (threadIdx.x == 0) {
         double s = 0.0;
         for (int k = 0; k < 8; k++) s += w[k];
         part[c] = s;
+        __threadfence();
+        is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
-}
-
-template <class Fin>
-__global__ void k_seg_finish(int n_sys, const int* __restrict__ chunk0, const double* __restrict__ part,
-                             Fin fin, const int* gate) {
-    if (gate && *(volatile const int*)gate == 0) return;
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n_sys) return;
-    double t = 0.0;
-    for (int c = chunk0[s]; c < chunk0[s + 1]; c++) t += part[c];
-    fin(s, t);
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    for (int s = wid; s < n_sys; s += 8) {
+        double u = 0.0;
+        const int ce = chunk0[s + 1];
+        for (int k = chunk0[s] + lane; k < ce; k += 32) u += __ldcg(part + k);
+        u = warp_sum(u);
+        if (lane == 0) fin(s, u);
+    }
+    if (threadIdx.x == 0) *ticket = 0u;
 }
 
 struct FinSPAp {
@@ -361,6 +380,8 @@ struct Batch {
     DevArray<int> seg, chunk_lo, chunk_hi, chunk0;
     int n_chunks = 0;
     DevArray<double> part, r, z, p, Ap, rt;
+    DevArray<unsigned> ticket;   // of the segmented dots (zero between them)
+    int lanes0 = 0;              // lanes a row of the outer FP64 products
     DevArray<double> sc;     // 6 n_sys scalars
     DevArray<int> si;        // n_sys active flags + breakdown
     SegScal S{};
@@ -401,12 +422,10 @@ struct Batch {
     template <class Fin>
     void seg_dot(const double* a, const double* b, Fin fin, const int* gate = nullptr,
                  bool skip_stopped = true) {
-        k_seg_partial<<<n_chunks, 256, 0, stream()>>>(chunk_lo.get(), chunk_hi.get(), a, b,
-                                                      part.get(), gate, chunk_sys.get(),
-                                                      gating && skip_stopped ? S.active : nullptr);
-        RB_CHECK_LAUNCH();
-        k_seg_finish<<<grid_for(n_sys, 128), 128, 0, stream()>>>(n_sys, chunk0.get(), part.get(),
-                                                                  fin, gate);
+        k_seg_dot<<<n_chunks, 256, 0, stream()>>>(chunk_lo.get(), chunk_hi.get(), a, b, part.get(),
+                                                  gate, chunk_sys.get(),
+                                                  gating && skip_stopped ? S.active : nullptr, n_sys,
+                                                  chunk0.get(), ticket.get(), fin);
         RB_CHECK_LAUNCH();
     }
 
@@ -638,6 +657,12 @@ void Batch::setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o) {
         chunk_sys.upload(cs.data(), cs.size());
     }
     part.alloc((size_t)n_chunks);
+    ticket.alloc(1);
+    ticket.zero();
+    // the outer products read the same rows as the cycle's finest level, on
+    // the width timed for it (9-point rows: 2 lanes; the 8 that the mean row
+    // length suggests took 24 us against 14 on half a million rows)
+    lanes0 = (o.precision == RB_PREC_FP32 ? cat.lv32[0].gA : cat.lv64[0].gA) & (kRowsBlocked - 1);
     seg.alloc((size_t)std::max<long long>(N, 1));
     DevArray<long long> offd((size_t)n + 1);
     offd.upload(off[0].data(), n + 1);
@@ -820,7 +845,7 @@ int Batch::pcg(double* x, const double* b, double tol, int max_iter, int* iters,
     if (cat.use_graphs) return pcg_device_loop(x, b, tol, max_iter, iters, relres, bnorm, restart);
     auto body = [&](bool full_r) {
         launch_rows(Av.rowptr, Av.cols, Av.vals, N, Av.nnz, p.get(),
-                    row_gate(EpiStore<double>{Ap.get()}, gate(0)), cat.gA0 > 0 ? cat.gA0 : 0);
+                    row_gate(EpiStore<double>{Ap.get()}, gate(0)), lanes0);
         seg_dot(p.get(), Ap.get(), FinSPAp{S});
         k_seg_update<<<grid_for(N, 256), 256, 0, stream()>>>(N, seg.get(), x, r.get(), p.get(),
                                                              Ap.get(), S.alpha, S.active);
@@ -828,7 +853,7 @@ int Batch::pcg(double* x, const double* b, double tol, int max_iter, int* iters,
         if (full_r)
             launch_rows(Av.rowptr, Av.cols, Av.vals, N, Av.nnz, x,
                         row_gate(EpiResidual<double, double>{b, r.get()}, gate(0)),
-                        cat.gA0 > 0 ? cat.gA0 : 0);
+                        lanes0);
         seg_dot(r.get(), r.get(), FinSRR{S});
         cycle64(z.get(), r.get());
         seg_dot(r.get(), z.get(), FinSRZ{S});
@@ -897,14 +922,14 @@ int Batch::pcg_device_loop(double* x, const double* b, double tol, int max_iter,
                                                             S.beta, C, S.active);
         RB_CHECK_LAUNCH();
         launch_rows(Av.rowptr, Av.cols, Av.vals, N, Av.nnz, p.get(),
-                    row_gate(EpiStore<double>{Ap.get()}, gate(0)), cat.gA0 > 0 ? cat.gA0 : 0);
+                    row_gate(EpiStore<double>{Ap.get()}, gate(0)), lanes0);
         seg_dot(p.get(), Ap.get(), FinSPAp{S});
         k_seg_update<<<grid_for(N, 256), 256, 0, stream()>>>(N, seg.get(), x, r.get(), p.get(),
                                                              Ap.get(), S.alpha, S.active);
         RB_CHECK_LAUNCH();
         launch_rows(Av.rowptr, Av.cols, Av.vals, N, Av.nnz, x,
                     row_gate(EpiResidualIf<double, double>{b, r.get(), &C->full}, gate(0)),
-                    cat.gA0 > 0 ? cat.gA0 : 0);
+                    lanes0);
         seg_dot(r.get(), r.get(), FinSRR{S});
         cycle64(z.get(), r.get());
         seg_dot(r.get(), z.get(), FinSRZ{S});
@@ -912,7 +937,7 @@ int Batch::pcg_device_loop(double* x, const double* b, double tol, int max_iter,
         RB_CHECK_LAUNCH();
         launch_rows(Av.rowptr, Av.cols, Av.vals, N, Av.nnz, x,
                     row_gate(EpiResidualIf<double, double>{b, rt.get(), &C->confirm}, gate(0)),
-                    cat.gA0 > 0 ? cat.gA0 : 0);
+                    lanes0);
         seg_dot(rt.get(), rt.get(), FinSTmp{S}, &C->confirm);
         k_batch_confirm<<<sg, 128, 0, stream()>>>(n, S, bnorm_d.get(), cand_d.get(),
                                                   iters_d.get(), relres_d.get(), C);
