@@ -743,115 +743,160 @@ __global__ void k_ext_fill(int n, const int* __restrict__ arp, const int* __rest
 // positions, and every sum whose order matters (col_sum, weak_sum, the
 // filter's row sums) is folded sequentially in the original order.  Rows
 // whose set exceeds kExtWarpMax entries take the one-thread-per-row kernels.
-constexpr int kExtHash = 2 * kExtWarpMax;   // hash slots per warp
+//
+// Rows whose set has at most kExtSmall entries (nearly all) use tables of that
+// size: 1.8 KB a warp, so the registers and not the shared memory bound the
+// warps an SM holds; the others use kExtWarpMax.  What a row reads of its
+// neighbours is loaded a lane a neighbour, and a neighbour's row one
+// neighbour ahead, so a warp waits on one memory round trip a neighbour and
+// not on the chain of four (index, state, row pointers, entries).
+constexpr int kExtSmall = 64;
 constexpr int kExtWarps = 8;                // warps per block
 
+template <int CAP>
 struct ExtWarpMem {
-    int keys[kExtHash];
-    int pos[kExtHash];
-    int list[kExtWarpMax];
-    double vals[kExtWarpMax];
+    static constexpr int H = 2 * CAP;       // hash slots
+    int keys[H];
+    int pos[H];
+    int list[CAP];
+    double vals[CAP];
 };
 
 __device__ __forceinline__ unsigned ext_hash(int c) { return (unsigned)c * 2654435761u; }
 
 // position of column c in the set, or -1
-__device__ __forceinline__ int ext_find(const ExtWarpMem& w, int c) {
-    unsigned h = ext_hash(c) & (kExtHash - 1);
+template <int CAP>
+__device__ __forceinline__ int ext_find(const ExtWarpMem<CAP>& w, int c) {
+    unsigned h = (ext_hash(c) >> 16) & (ExtWarpMem<CAP>::H - 1);
     while (true) {
         const int k = w.keys[h];
         if (k == c) return w.pos[h];
         if (k == -1) return -1;
-        h = (h + 1) & (kExtHash - 1);
+        h = (h + 1) & (ExtWarpMem<CAP>::H - 1);
     }
 }
 
 // insert column c (not yet present) at position p; distinct keys may be
 // inserted by several lanes at once
-__device__ __forceinline__ void ext_insert(ExtWarpMem& w, int c, int p) {
-    unsigned h = ext_hash(c) & (kExtHash - 1);
+template <int CAP>
+__device__ __forceinline__ void ext_insert(ExtWarpMem<CAP>& w, int c, int p) {
+    unsigned h = (ext_hash(c) >> 16) & (ExtWarpMem<CAP>::H - 1);
     while (true) {
         if (atomicCAS(&w.keys[h], -1, c) == -1) {
             w.pos[h] = p;
             return;
         }
-        h = (h + 1) & (kExtHash - 1);
+        h = (h + 1) & (ExtWarpMem<CAP>::H - 1);
     }
 }
 
-// Insertion-ordered C set of row i; returns its size, or kExtWarpMax + 1
-// when it does not fit.
+// cs[k] = the column of S's entry k when it is a C point, else -1 (the
+// pattern only asks for the C points of a neighbour's row)
+__global__ void k_ext_cflag(long long nnz, const int* __restrict__ sci, const int* __restrict__ st,
+                            int* __restrict__ cs) {
+    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nnz) return;
+    const int c = sci[k];
+    cs[k] = st[c] == kSelected ? c : -1;
+}
+
+// Insertion-ordered C set of row i; returns its size, or CAP + 1 when it
+// does not fit.
+template <int CAP>
 __device__ int ext_build_warp(int i, const int* __restrict__ srp, const int* __restrict__ sci,
-                              const int* __restrict__ st, ExtWarpMem& w, int lane) {
-    for (int t = lane; t < kExtHash; t += 32) w.keys[t] = -1;
+                              const int* __restrict__ cs, const int* __restrict__ st,
+                              ExtWarpMem<CAP>& w, int lane) {
+    for (int t = lane; t < ExtWarpMem<CAP>::H; t += 32) w.keys[t] = -1;
     __syncwarp();
     int m = 0;
-    for (int j = srp[i] + 1; j < srp[i + 1]; j++) {
-        const int c = sci[j];
-        const int sc = st[c];
-        if (sc == kSelected) {
-            if (ext_find(w, c) < 0) {
-                if (m >= kExtWarpMax) return kExtWarpMax + 1;
-                if (lane == 0) {
-                    w.list[m] = c;
-                    ext_insert(w, c, m);
-                }
-                m++;
-                __syncwarp();
+    const int s1 = srp[i + 1];
+    for (int j0 = srp[i] + 1; j0 < s1; j0 += 32) {
+        // a lane a neighbour: its column, state and row
+        const int nb = min(32, s1 - j0);
+        int c = 0, sc = kNoNeighbors, b = 0, e = 0;
+        if (lane < nb) {
+            c = sci[j0 + lane];
+            sc = st[c];
+            if (sc == kUnselected) { b = srp[c] + 1; e = srp[c + 1]; }
+        }
+        int bt = __shfl_sync(0xffffffffu, b, 0), et = __shfl_sync(0xffffffffu, e, 0);
+        int next = bt + lane < et ? cs[bt + lane] : -1;   // first entries of neighbour t
+        for (int t = 0; t < nb; t++) {
+            const int ct = __shfl_sync(0xffffffffu, c, t), st_t = __shfl_sync(0xffffffffu, sc, t);
+            const int cur = next, bc = bt, ec = et;
+            if (t + 1 < nb) {
+                bt = __shfl_sync(0xffffffffu, b, t + 1);
+                et = __shfl_sync(0xffffffffu, e, t + 1);
+                next = bt + lane < et ? cs[bt + lane] : -1;
             }
-        } else if (sc == kUnselected) {
-            for (int base = srp[c] + 1; base < srp[c + 1]; base += 32) {
-                const int k = base + lane;
-                const int ck = k < srp[c + 1] ? sci[k] : -1;
-                const bool isnew = ck >= 0 && st[ck] == kSelected && ext_find(w, ck) < 0;
-                const unsigned b = __ballot_sync(0xffffffffu, isnew);
-                const int add = __popc(b);
-                if (m + add > kExtWarpMax) return kExtWarpMax + 1;
-                if (isnew) {
-                    const int p = m + __popc(b & ((1u << lane) - 1));
-                    w.list[p] = ck;
-                    ext_insert(w, ck, p);
+            if (st_t == kSelected) {
+                if (ext_find(w, ct) < 0) {
+                    if (m >= CAP) return CAP + 1;
+                    if (lane == 0) {
+                        w.list[m] = ct;
+                        ext_insert(w, ct, m);
+                    }
+                    m++;
+                    __syncwarp();
                 }
-                m += add;
-                __syncwarp();
+            } else if (st_t == kUnselected) {
+                for (int base = bc; base < ec; base += 32) {
+                    const int ck = base == bc ? cur : (base + lane < ec ? cs[base + lane] : -1);
+                    const bool isnew = ck >= 0 && ext_find(w, ck) < 0;
+                    const unsigned bal = __ballot_sync(0xffffffffu, isnew);
+                    const int add = __popc(bal);
+                    if (m + add > CAP) return CAP + 1;
+                    if (isnew) {
+                        const int p = m + __popc(bal & ((1u << lane) - 1));
+                        w.list[p] = ck;
+                        ext_insert(w, ck, p);
+                    }
+                    m += add;
+                    __syncwarp();
+                }
             }
         }
     }
     return m;
 }
 
-// Pattern sizes of the rows whose C set fits; a row that does not is marked
-// (big[i] = 1) for the one-thread-per-row kernel.
+// Pattern sizes of the rows whose C set fits.  big[i]: 0 counted, 2 larger
+// than kExtSmall (the kExtWarpMax pass looks at those only), 1 larger than
+// kExtWarpMax (the one-thread-per-row kernel counts it).
+template <int CAP>
 __global__ void __launch_bounds__(kExtWarps * 32)
 k_ext_pattern_warp(int n, const int* __restrict__ srp, const int* __restrict__ sci,
-                   const int* __restrict__ st, int* cnt, int* big) {
+                   const int* __restrict__ cs, const int* __restrict__ st, int* cnt, int* big) {
     extern __shared__ unsigned char ext_smem[];
-    ExtWarpMem& w = reinterpret_cast<ExtWarpMem*>(ext_smem)[threadIdx.x >> 5];
+    ExtWarpMem<CAP>& w = reinterpret_cast<ExtWarpMem<CAP>*>(ext_smem)[threadIdx.x >> 5];
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= n) return;
+    if (CAP != kExtSmall && big[i] != 2) return;
     if (st[i] != kUnselected) {
         if (lane == 0) { cnt[i] = st[i] == kSelected ? 1 : 0; big[i] = 0; }
         return;
     }
-    const int m = ext_build_warp(i, srp, sci, st, w, lane);
+    const int m = ext_build_warp<CAP>(i, srp, sci, cs, st, w, lane);
     if (lane == 0) {
-        big[i] = m > kExtWarpMax ? 1 : 0;
-        if (m <= kExtWarpMax) cnt[i] = m;
+        big[i] = m <= CAP ? 0 : CAP == kExtSmall ? 2 : 1;
+        if (m <= CAP) cnt[i] = m;
     }
 }
 
+// Rows of 1 .. kExtSmall entries (CAP = kExtSmall) or of more, up to CAP.
+template <int CAP>
 __global__ void __launch_bounds__(kExtWarps * 32)
 k_ext_fill_warp(int n, const int* __restrict__ arp, const int* __restrict__ aci,
                 const double* __restrict__ acv, const int* __restrict__ srp,
-                const int* __restrict__ sci, const int* __restrict__ st,
-                const int* __restrict__ prp, int* pcols, double* pvals, double filter,
-                int* kept, const int* __restrict__ nv) {
+                const int* __restrict__ sci, const int* __restrict__ cs,
+                const int* __restrict__ st, const int* __restrict__ prp, int* pcols,
+                double* pvals, double filter, int* kept, const int* __restrict__ nv) {
     extern __shared__ unsigned char ext_smem[];
-    ExtWarpMem& w = reinterpret_cast<ExtWarpMem*>(ext_smem)[threadIdx.x >> 5];
+    ExtWarpMem<CAP>& w = reinterpret_cast<ExtWarpMem<CAP>*>(ext_smem)[threadIdx.x >> 5];
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= n) return;
     const int p0 = prp[i], p1 = prp[i + 1];
-    if (p1 - p0 > kExtWarpMax) return;   // the one-thread-per-row kernel takes it
+    if (p1 - p0 > CAP || (CAP != kExtSmall && p1 - p0 <= kExtSmall)) return;
     const int si = st[i];
     int m = 0;
     if (si == kSelected) {
@@ -859,75 +904,126 @@ k_ext_fill_warp(int n, const int* __restrict__ arp, const int* __restrict__ aci,
         m = 1;
         __syncwarp();
     } else if (si == kUnselected) {
-        m = ext_build_warp(i, srp, sci, st, w, lane);
+        m = ext_build_warp<CAP>(i, srp, sci, cs, st, w, lane);
         for (int t = lane; t < m; t += 32) w.vals[t] = 0.0;
         __syncwarp();
         int start = arp[i];
         const int end = arp[i + 1];
         double weak_sum = acv[start++];
-        int ctr = srp[i] + 1;
-        const int end_S = srp[i + 1];
-        for (int j = start; j < end; j++) {
-            const int col = aci[j];
-            const double val = acv[j];
-            const int idx = ext_find(w, col);
-            if (idx >= 0) {
-                if (lane == 0) w.vals[idx] = dadd(w.vals[idx], val);
-                __syncwarp();
-                if (ctr < end_S && sci[ctr] == col) ctr++;
-            } else if (ctr < end_S && sci[ctr] == col) {
-                ctr++;
-                if (st[col] != kUnselected) continue;
-                const int sk = arp[col] + 1, ek = arp[col + 1];
-                const int sign = acv[arp[col]] > 0 ? 1 : -1;
+        // the strong neighbours, a lane each (the first 32; later ones are read)
+        const int s0 = srp[i] + 1, end_S = srp[i + 1];
+        const int scol = s0 + lane < end_S ? sci[s0 + lane] : -1;
+        int ctr = s0;
+        for (int j0 = start; j0 < end; j0 += 32) {
+            // a lane an entry of row i: its column's state, place in the set
+            // (the set does not change any more), row and diagonal's sign
+            const int nb = min(32, end - j0);
+            int col = 0, stc = kNoNeighbors, idx = -1, ab = 0, ae = 0, sign = 0;
+            double val = 0.0;
+            if (lane < nb) {
+                col = aci[j0 + lane];
+                val = acv[j0 + lane];
+                stc = st[col];
+                idx = ext_find(w, col);
+                if (stc == kUnselected) {
+                    ab = arp[col] + 1;
+                    ae = arp[col + 1];
+                    sign = ae >= ab && acv[ab - 1] > 0 ? 1 : -1;
+                }
+            }
+            int bt = __shfl_sync(0xffffffffu, ab, 0), et = __shfl_sync(0xffffffffu, ae, 0);
+            int nc = -1;
+            double nval = 0.0;
+            if (bt + lane < et) { nc = aci[bt + lane]; nval = acv[bt + lane]; }
+            for (int t = 0; t < nb; t++) {
+                const int bc = bt, ec = et;
+                const int cc = nc;
+                const double cval = nval;
+                if (t + 1 < nb) {
+                    bt = __shfl_sync(0xffffffffu, ab, t + 1);
+                    et = __shfl_sync(0xffffffffu, ae, t + 1);
+                    nc = -1;
+                    nval = 0.0;
+                    if (bt + lane < et) { nc = aci[bt + lane]; nval = acv[bt + lane]; }
+                }
+                const int colt = __shfl_sync(0xffffffffu, col, t);
+                const int idt = __shfl_sync(0xffffffffu, idx, t);
+                const double valt = __shfl_sync(0xffffffffu, val, t);
+                int sc_at = -1;
+                if (ctr < end_S) {
+                    const int o = ctr - s0;
+                    sc_at = o < 32 ? __shfl_sync(0xffffffffu, scol, o) : sci[ctr];
+                }
+                const bool strong = ctr < end_S && sc_at == colt;
+                if (strong) ctr++;
+                if (idt >= 0) {
+                    if (lane == 0) w.vals[idt] = dadd(w.vals[idt], valt);
+                    __syncwarp();
+                    continue;
+                }
+                const int stt = __shfl_sync(0xffffffffu, stc, t);
+                if (!strong) {
+                    if (stt != kNoNeighbors && same_var(i, colt, nv)) weak_sum = dadd(weak_sum, valt);
+                    continue;
+                }
+                if (stt != kUnselected) continue;
+                const double sg = (double)__shfl_sync(0xffffffffu, sign, t);
                 // col_sum: the qualifying entries of row col, summed in order
+                // (an entry that does not qualify adds +0, which changes no
+                // sum that starts at +0)
                 double col_sum = 0;
-                for (int base = sk; base < ek; base += 32) {
+                int id = -1;   // of the first 32 entries, kept for the expansion
+                bool neg = false;
+                for (int base = bc; base < ec; base += 32) {
                     const int k = base + lane;
                     double vk = 0.0;
                     bool q = false;
-                    if (k < ek) {
-                        vk = acv[k];
-                        const int ck = aci[k];
-                        q = dmul(vk, (double)sign) < 0 && (ck == i || ext_find(w, ck) >= 0);
+                    if (k < ec) {
+                        vk = base == bc ? cval : acv[k];
+                        const int ck = base == bc ? cc : aci[k];
+                        const bool ng = dmul(vk, sg) < 0;
+                        int f = -1;
+                        if (ng) f = ck == i ? 0 : ext_find(w, ck);
+                        q = ng && f >= 0;
+                        if (base == bc) { id = f; neg = ng; }
                     }
-                    unsigned b = __ballot_sync(0xffffffffu, q);
-                    while (b) {
-                        const int t = __ffs(b) - 1;
-                        col_sum = dadd(col_sum, __shfl_sync(0xffffffffu, vk, t));
-                        b &= b - 1;
+                    const double vq = q ? vk : 0.0;
+                    const int cnt = min(32, ec - base);
+                    for (int u0 = 0; u0 < cnt; u0 += 8) {
+#pragma unroll
+                        for (int u = 0; u < 8; u++)
+                            col_sum = dadd(col_sum, __shfl_sync(0xffffffffu, vq, u0 + u));
                     }
                 }
                 if (fabs(col_sum) < kZeroTol) {
-                    weak_sum = dadd(weak_sum, val);
-                } else {
-                    col_sum = __ddiv_rn(val, col_sum);
-                    for (int base = sk; base < ek; base += 32) {
-                        const int k = base + lane;
-                        bool self = false;
-                        double term = 0.0;
-                        if (k < ek) {
-                            const int ck = aci[k];
-                            const double vk = acv[k];
-                            if (dmul(vk, (double)sign) < 0) {
-                                term = dmul(col_sum, vk);
-                                if (ck == i) {
-                                    self = true;
-                                } else {
-                                    const int id = ext_find(w, ck);
-                                    if (id >= 0) w.vals[id] = dadd(w.vals[id], term);
-                                }
+                    weak_sum = dadd(weak_sum, valt);
+                    continue;
+                }
+                col_sum = __ddiv_rn(valt, col_sum);
+                for (int base = bc; base < ec; base += 32) {
+                    const int k = base + lane;
+                    bool self = false;
+                    double term = 0.0;
+                    if (k < ec) {
+                        const int ck = base == bc ? cc : aci[k];
+                        const double vk = base == bc ? cval : acv[k];
+                        const bool ng = base == bc ? neg : dmul(vk, sg) < 0;
+                        if (ng) {
+                            term = dmul(col_sum, vk);
+                            if (ck == i) {
+                                self = true;
+                            } else {
+                                const int f = base == bc ? id : ext_find(w, ck);
+                                if (f >= 0) w.vals[f] = dadd(w.vals[f], term);
                             }
                         }
-                        // i occurs at most once in row col: its term joins
-                        // weak_sum at its place in the sequence
-                        const unsigned sb = __ballot_sync(0xffffffffu, self);
-                        if (sb) weak_sum = dadd(weak_sum, __shfl_sync(0xffffffffu, term, __ffs(sb) - 1));
                     }
-                    __syncwarp();
+                    // i occurs at most once in row col: its term joins
+                    // weak_sum at its place in the sequence
+                    const unsigned sb = __ballot_sync(0xffffffffu, self);
+                    if (sb) weak_sum = dadd(weak_sum, __shfl_sync(0xffffffffu, term, __ffs(sb) - 1));
                 }
-            } else {
-                if (st[col] != kNoNeighbors && same_var(i, col, nv)) weak_sum = dadd(weak_sum, val);
+                __syncwarp();
             }
         }
         if (fabs(weak_sum) > kZeroTol)
@@ -1053,14 +1149,24 @@ rb_csr_s* interpolation(const rb_csr_s& A, const rb_csr_s& S, const int* st, int
     if (n) k_ext_bound<<<g, 256, 0, stream()>>>(n, S.rowptr.get(), S.cols.get(), st, ub.get());
     RB_CHECK_LAUNCH();
     DevArray<int> big((size_t)n + 1);
-    RB_CUDA(cudaFuncSetAttribute(k_ext_pattern_warp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(kExtWarps * sizeof(ExtWarpMem))));
-    RB_CUDA(cudaFuncSetAttribute(k_ext_fill_warp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(kExtWarps * sizeof(ExtWarpMem))));
-    if (n)
-        k_ext_pattern_warp<<<grid_for((long)n * 32, kExtWarps * 32), kExtWarps * 32,
-                             kExtWarps * sizeof(ExtWarpMem), stream()>>>(
-            n, S.rowptr.get(), S.cols.get(), st, cnt.get(), big.get());
+    DevArray<int> cs((size_t)std::max<long long>(S.nnz, 1));
+    if (S.nnz)
+        k_ext_cflag<<<grid_for(S.nnz, 256), 256, 0, stream()>>>(S.nnz, S.cols.get(), st, cs.get());
+    RB_CHECK_LAUNCH();
+    const unsigned gw = grid_for((long)n * 32, kExtWarps * 32);
+    constexpr size_t smem_small = kExtWarps * sizeof(ExtWarpMem<kExtSmall>);
+    constexpr size_t smem_large = kExtWarps * sizeof(ExtWarpMem<kExtWarpMax>);
+    RB_CUDA(cudaFuncSetAttribute(k_ext_pattern_warp<kExtWarpMax>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_large));
+    RB_CUDA(cudaFuncSetAttribute(k_ext_fill_warp<kExtWarpMax>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_large));
+    if (n) {
+        k_ext_pattern_warp<kExtSmall><<<gw, kExtWarps * 32, smem_small, stream()>>>(
+            n, S.rowptr.get(), S.cols.get(), cs.get(), st, cnt.get(), big.get());
+        RB_CHECK_LAUNCH();
+        k_ext_pattern_warp<kExtWarpMax><<<gw, kExtWarps * 32, smem_large, stream()>>>(
+            n, S.rowptr.get(), S.cols.get(), cs.get(), st, cnt.get(), big.get());
+    }
     RB_CHECK_LAUNCH();
     std::vector<int> ubh((size_t)n), bigh((size_t)n);
     ub.download(ubh.data(), n);
@@ -1102,10 +1208,13 @@ rb_csr_s* interpolation(const rb_csr_s& A, const rb_csr_s& S, const int* st, int
     pcols.alloc((size_t)std::max(nnz0, 1LL));
     pvals.alloc((size_t)std::max(nnz0, 1LL));
     if (n) {
-        k_ext_fill_warp<<<grid_for((long)n * 32, kExtWarps * 32), kExtWarps * 32,
-                          kExtWarps * sizeof(ExtWarpMem), stream()>>>(
-            n, A.rowptr.get(), A.cols.get(), A.vals.get(), S.rowptr.get(), S.cols.get(), st,
-            prp.get(), pcols.get(), pvals.get(), filter, kept.get(), nv);
+        k_ext_fill_warp<kExtSmall><<<gw, kExtWarps * 32, smem_small, stream()>>>(
+            n, A.rowptr.get(), A.cols.get(), A.vals.get(), S.rowptr.get(), S.cols.get(), cs.get(),
+            st, prp.get(), pcols.get(), pvals.get(), filter, kept.get(), nv);
+        RB_CHECK_LAUNCH();
+        k_ext_fill_warp<kExtWarpMax><<<gw, kExtWarps * 32, smem_large, stream()>>>(
+            n, A.rowptr.get(), A.cols.get(), A.vals.get(), S.rowptr.get(), S.cols.get(), cs.get(),
+            st, prp.get(), pcols.get(), pvals.get(), filter, kept.get(), nv);
         RB_CHECK_LAUNCH();
         k_ext_fill<<<g, 256, 0, stream()>>>(
             n, A.rowptr.get(), A.cols.get(), A.vals.get(), S.rowptr.get(), S.cols.get(), st,
@@ -1132,7 +1241,12 @@ rb_csr_s* interpolation(const rb_csr_s& A, const rb_csr_s& S, const int* st, int
 // dropped; the row is written sorted by column (add_append's sort,
 // util/linalg/add.cpp:75).  Pass 1 counts survivors, pass 2 writes them.
 
-__device__ __forceinline__ unsigned hash_col(int c) { return (unsigned)c * 2654435761u; }
+// (the upper bits folded in: the low bits of the product alone depend on the
+// low bits of c alone, and a product row's columns lie in runs a plane apart)
+__device__ __forceinline__ unsigned hash_col(int c) {
+    const unsigned h = (unsigned)c * 2654435761u;
+    return h ^ (h >> 16);
+}
 
 // Insert/find column c in an open-addressing table of size H (power of two).
 __device__ __forceinline__ int hash_slot(int* keys, int H, int c) {
@@ -1148,7 +1262,6 @@ __device__ __forceinline__ int hash_slot(int* keys, int H, int c) {
     }
 }
 
-template <bool WRITE>
 __device__ void spgemm_row(int lane, int row, const int* __restrict__ arp,
                            const int* __restrict__ aci, const double* __restrict__ acv,
                            const int* __restrict__ brp, const int* __restrict__ bci,
@@ -1178,8 +1291,7 @@ __device__ void spgemm_row(int lane, int row, const int* __restrict__ arp,
         m += __popc(bal);
     }
     __syncwarp();
-    if (lane == 0 && cnt) cnt[row] = m;
-    if (!WRITE) return;
+    if (lane == 0) cnt[row] = m;
     // rank by column and write sorted
     const int out = crp[row];
     for (int a = lane; a < m; a += 32) {
@@ -1193,8 +1305,7 @@ __device__ void spgemm_row(int lane, int row, const int* __restrict__ arp,
 }
 
 // Structural size of a row of C (distinct columns, before the |v| <= 1e-16
-// drop) with key-only hash tables: 4 bytes a slot instead of 16, so four
-// times the warps per SM of the numeric pass.
+// drop) with a key-only hash table (tables in global scratch, one warp a row).
 __device__ void spgemm_row_keys(int lane, int row, const int* __restrict__ arp,
                                 const int* __restrict__ aci, const int* __restrict__ brp,
                                 const int* __restrict__ bci, int* keys, int H, int* scnt) {
@@ -1213,16 +1324,174 @@ __device__ void spgemm_row_keys(int lane, int row, const int* __restrict__ arp,
     if (lane == 0) scnt[row] = m;
 }
 
-template <int H, int WPB>
+// ---- rows in shared tables, G lanes a row ------------------------------
+// 32 / G rows share a warp (G = 8 where B's rows are short, as the
+// prolongator's: with a whole warp a row, 4 of 32 lanes had an entry).  A
+// group's A entries are loaded a lane an entry with the bounds of their B
+// rows, and the first entries of the next B row before the current one is
+// used, so a step waits on shared memory only.  The loops run to the longest
+// row of the warp (entries past a row's end are predicated off), so that the
+// groups stay together; within a group the A entries are taken one after
+// another with a warp barrier between, so every sum receives its terms in
+// A's row order.
+//
+// step(value of the A entry, column of the B entry or -1, its value) is
+// called for every entry by the lane that holds it.
+template <int G, bool VALS, class Step>
+__device__ __forceinline__ void spgemm_walk(int gl, int as, int ae, const int* __restrict__ aci,
+                                            const double* __restrict__ acv,
+                                            const int* __restrict__ brp,
+                                            const int* __restrict__ bci,
+                                            const double* __restrict__ bcv, Step step) {
+    const int L = (int)__reduce_max_sync(0xffffffffu, (unsigned)(ae - as));
+    for (int j0 = 0; j0 < L; j0 += G) {
+        int bs = 0, be = 0;
+        double va = 0.0;
+        if (as + j0 + gl < ae) {
+            const int ca = aci[as + j0 + gl];
+            bs = brp[ca];
+            be = brp[ca + 1];
+            if (VALS) va = acv[as + j0 + gl];
+        }
+        const int nt = min(G, L - j0);
+        int b1 = __shfl_sync(0xffffffffu, bs, 0, G), e1 = __shfl_sync(0xffffffffu, be, 0, G);
+        int nc = -1;
+        double nv = 0.0;
+        if (b1 + gl < e1) {
+            nc = bci[b1 + gl];
+            if (VALS) nv = bcv[b1 + gl];
+        }
+        for (int t = 0; t < nt; t++) {
+            const int b0 = b1, e0 = e1;
+            const double vt = VALS ? __shfl_sync(0xffffffffu, va, t, G) : 0.0;
+            int cc = nc;
+            double cv = nv;
+            if (t + 1 < nt) {
+                b1 = __shfl_sync(0xffffffffu, bs, t + 1, G);
+                e1 = __shfl_sync(0xffffffffu, be, t + 1, G);
+                nc = -1;
+                if (b1 + gl < e1) {
+                    nc = bci[b1 + gl];
+                    if (VALS) nv = bcv[b1 + gl];
+                }
+            }
+            const int nq = ((int)__reduce_max_sync(0xffffffffu, (unsigned)(e0 - b0)) + G - 1) / G;
+            for (int q = 0; q < nq; q++) {
+                if (q) {
+                    const int k = b0 + q * G + gl;
+                    cc = k < e0 ? bci[k] : -1;
+                    if (VALS && k < e0) cv = bcv[k];
+                }
+                step(vt, cc, cv);
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// Distinct columns of each listed row (rows NULL: rows 0 .. nrows - 1) in a
+// table of H keys; a row with more than 3/4 H of them stops counting and goes
+// to the list `over`.
+template <int G, int H, int WPB>
 __global__ void __launch_bounds__(WPB * 32)
 k_spgemm_keys(const int* __restrict__ rows, int nrows, const int* __restrict__ arp,
               const int* __restrict__ aci, const int* __restrict__ brp,
-              const int* __restrict__ bci, int* scnt) {
+              const int* __restrict__ bci, int* scnt, int* over, int* over_count) {
     extern __shared__ int kmem[];
+    constexpr int RPW = 32 / G, LIMIT = H / 4 * 3;
+    static_assert(LIMIT + G < H, "a probe always meets a free slot");
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int idx = blockIdx.x * WPB + w;
-    if (idx >= nrows) return;
-    spgemm_row_keys(lane, rows[idx], arp, aci, brp, bci, kmem + (size_t)w * H, H, scnt);
+    const int gl = lane & (G - 1), sub = lane / G;
+    const long idx = ((long)blockIdx.x * WPB + w) * RPW + sub;
+    if (((long)blockIdx.x * WPB + w) * RPW >= nrows) return;
+    const bool valid = idx < nrows;
+    const int row = valid ? (rows ? rows[idx] : (int)idx) : 0;
+    int* keys = kmem + ((size_t)w * RPW + sub) * H;
+    for (int t = gl; t < H; t += G) keys[t] = -1;
+    __syncwarp();
+    const unsigned gbits = (G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u)) << (lane & ~(G - 1));
+    int count = 0;
+    spgemm_walk<G, false>(gl, valid ? arp[row] : 0, valid ? arp[row + 1] : 0, aci, nullptr, brp,
+                          bci, nullptr, [&](double, int c, double) {
+        bool fresh = false;
+        if (c >= 0 && count <= LIMIT) {
+            unsigned h = hash_col(c) & (H - 1);
+            while (true) {
+                const int k = keys[h];
+                if (k == c) break;
+                if (k == -1) {
+                    const int old = atomicCAS(keys + h, -1, c);
+                    if (old == -1) { fresh = true; break; }
+                    if (old == c) break;
+                }
+                h = (h + 1) & (H - 1);
+            }
+        }
+        count += __popc(__ballot_sync(0xffffffffu, fresh) & gbits);
+    });
+    if (gl == 0 && valid) {
+        if (count <= LIMIT) scnt[row] = count;
+        else over[atomicAdd(over_count, 1)] = row;
+    }
+}
+
+// The listed rows' entries in tables of H slots (at most H / 2 distinct
+// columns): sums in A's row order, |v| <= 1e-16 dropped, written sorted by
+// column at crp[row]; cnt[row] = entries kept.
+template <int G, int H, int WPB>
+__global__ void __launch_bounds__(WPB * 32)
+k_spgemm_smem(const int* __restrict__ rows, int nrows, const int* __restrict__ arp,
+              const int* __restrict__ aci, const double* __restrict__ acv,
+              const int* __restrict__ brp, const int* __restrict__ bci,
+              const double* __restrict__ bcv, int* cnt, const int* crp, int* cci, double* ccv) {
+    extern __shared__ unsigned char smem[];
+    constexpr int RPW = 32 / G;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int gl = lane & (G - 1), sub = lane / G;
+    const long first = ((long)blockIdx.x * WPB + w) * RPW;
+    if (first >= nrows) return;
+    const bool valid = first + sub < nrows;
+    const int row = valid ? rows[first + sub] : 0;
+    double* sums = reinterpret_cast<double*>(smem) + ((size_t)w * RPW + sub) * H;
+    int* keys = reinterpret_cast<int*>(reinterpret_cast<double*>(smem) + (size_t)WPB * RPW * H) +
+                ((size_t)w * RPW + sub) * H;
+    for (int t = gl; t < H; t += G) { keys[t] = -1; sums[t] = 0.0; }
+    __syncwarp();
+    spgemm_walk<G, true>(gl, valid ? arp[row] : 0, valid ? arp[row + 1] : 0, aci, acv, brp, bci, bcv,
+                         [&](double va, int c, double vb) {
+        if (c >= 0) {
+            const int slot = hash_slot(keys, H, c);
+            sums[slot] = dadd(sums[slot], dmul(va, vb));
+        }
+    });
+    // the survivors moved to the table's front (a survivor's place is never
+    // past its slot, and a step's slots are read before any is written)
+    int m = 0;
+    for (int base = 0; base < H; base += G) {
+        const int k = keys[base + gl];
+        const double v = sums[base + gl];
+        const bool keep = k != -1 && fabs(v) > kZeroTol;
+        const unsigned bal = __ballot_sync(0xffffffffu, keep) >> (lane & ~(G - 1));
+        const unsigned mine = G == 32 ? bal : bal & ((1u << (G & 31)) - 1u);
+        if (keep) {
+            const int p = m + __popc(mine & ((1u << gl) - 1u));
+            keys[p] = k;
+            sums[p] = v;
+        }
+        m += __popc(mine);
+        __syncwarp();
+    }
+    if (!valid) return;
+    if (gl == 0) cnt[row] = m;
+    // rank by column and write sorted
+    const int out = crp[row];
+    for (int e = gl; e < m; e += G) {
+        const int c = keys[e];
+        int r = 0;
+        for (int q = 0; q < m; q++) r += keys[q] < c;
+        cci[out + r] = c;
+        ccv[out + r] = sums[e];
+    }
 }
 
 __global__ void k_spgemm_keys_global(const int* __restrict__ rows, int nrows,
@@ -1235,15 +1504,30 @@ __global__ void k_spgemm_keys_global(const int* __restrict__ rows, int nrows,
     spgemm_row_keys(lane, rows[w], arp, aci, brp, bci, gkeys + toff[w], tsize[w], scnt);
 }
 
-// Bin rows by a size: <= lim0 -> bin 0, <= lim1 -> bin 1, else bin 2.
-__global__ void k_bin_rows(int n, const int* __restrict__ size, int lim0, int lim1, int* bins,
+// Rows listed by a size into kBins lists of n places: bin b takes the sizes
+// up to lim[b] that no earlier bin takes, the last bin the rest.  A block
+// reserves its places in each list at once (a thread a counter update took
+// 0.17 ms on 262k rows).  The order inside a list does not matter.
+constexpr int kBins = 4;
+struct BinLimits { int lim[kBins - 1]; };
+__global__ void k_bin_rows(int n, const int* __restrict__ size, BinLimits lim, int* bins,
                            int* bin_count) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int u = size[i];
-    const int bin = u <= lim0 ? 0 : (u <= lim1 ? 1 : 2);
-    const int p = atomicAdd(bin_count + bin, 1);
-    bins[(size_t)bin * n + p] = i;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool valid = i < n;
+    __shared__ int local[kBins], start[kBins];
+    if (threadIdx.x < kBins) local[threadIdx.x] = 0;
+    __syncthreads();
+    int bin = 0, p = 0;
+    if (valid) {
+        const int u = size[i];
+        while (bin < kBins - 1 && u > lim.lim[bin]) bin++;
+        p = atomicAdd(&local[bin], 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < kBins && local[threadIdx.x])
+        start[threadIdx.x] = atomicAdd(bin_count + threadIdx.x, local[threadIdx.x]);
+    __syncthreads();
+    if (valid) bins[(size_t)bin * n + start[bin] + p] = i;
 }
 
 // Move each row's first cnt[i] entries from the capacity layout (cap
@@ -1260,25 +1544,7 @@ __global__ void k_spgemm_compact(int n, const int* __restrict__ cap, const int* 
     }
 }
 
-template <bool WRITE, int H, int WPB>
-__global__ void __launch_bounds__(WPB * 32)
-k_spgemm_smem(const int* __restrict__ rows, int nrows, const int* __restrict__ arp,
-              const int* __restrict__ aci, const double* __restrict__ acv,
-              const int* __restrict__ brp, const int* __restrict__ bci,
-              const double* __restrict__ bcv, int* cnt, const int* crp, int* cci, double* ccv) {
-    extern __shared__ unsigned char smem[];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double* sums = reinterpret_cast<double*>(smem) + (size_t)w * H;
-    int* keys = reinterpret_cast<int*>(reinterpret_cast<double*>(smem) + (size_t)WPB * H) + (size_t)w * 2 * H;
-    int* clist = keys + H;
-    const int idx = blockIdx.x * WPB + w;
-    if (idx >= nrows) return;
-    spgemm_row<WRITE>(lane, rows[idx], arp, aci, acv, brp, bci, bcv, keys, sums, clist, H, cnt,
-                      crp, cci, ccv);
-}
-
 // Rows whose bound exceeds the shared tables: tables in global scratch.
-template <bool WRITE>
 __global__ void k_spgemm_global(const int* __restrict__ rows, int nrows,
                                 const long long* __restrict__ toff, const int* __restrict__ tsize,
                                 const int* __restrict__ arp, const int* __restrict__ aci,
@@ -1289,28 +1555,31 @@ __global__ void k_spgemm_global(const int* __restrict__ rows, int nrows,
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (w >= nrows) return;
     const long long o = toff[w];
-    spgemm_row<WRITE>(lane, rows[w], arp, aci, acv, brp, bci, bcv, gkeys + o, gsums + o, glist + o,
+    spgemm_row(lane, rows[w], arp, aci, acv, brp, bci, bcv, gkeys + o, gsums + o, glist + o,
                       tsize[w], cnt, crp, cci, ccv);
 }
 
-// Upper bound of the row size of C and the bin of each row.
+// Upper bound of the row size of C.
 __global__ void k_spgemm_bound(int n, const int* __restrict__ arp, const int* __restrict__ aci,
-                               const int* __restrict__ brp, int* ub, int* bins, int* bin_count,
-                               int lim0, int lim1) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+                               const int* __restrict__ brp, int* ub) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     long long b = 0;
-    for (int j = arp[i]; j < arp[i + 1]; j++) b += brp[aci[j] + 1] - brp[aci[j]];
-    int u = (int)(b > INT_MAX / 4 ? INT_MAX / 4 : b);
-    ub[i] = u;
-    int bin = u <= lim0 ? 0 : (u <= lim1 ? 1 : 2);
-    int p = atomicAdd(bin_count + bin, 1);
-    bins[(size_t)bin * n + p] = i;
+    if (i < n) {
+        int j = arp[i];
+        const int e = arp[i + 1];
+        for (; j + 4 <= e; j += 4) {
+            int c[4], l[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) c[q] = aci[j + q];
+#pragma unroll
+            for (int q = 0; q < 4; q++) l[q] = brp[c[q] + 1] - brp[c[q]];
+#pragma unroll
+            for (int q = 0; q < 4; q++) b += l[q];
+        }
+        for (; j < e; j++) b += brp[aci[j] + 1] - brp[aci[j]];
+    }
+    if (i < n) ub[i] = (int)(b > INT_MAX / 4 ? INT_MAX / 4 : b);
 }
-
-namespace {
-constexpr int kH0 = 512, kW0 = 8;    // 8 warps x (512 x 16 B) = 64 KB
-constexpr int kH1 = 4096, kW1 = 2;   // 2 warps x (4096 x 16 B) = 128 KB
 
 inline int next_pow2(int v) {
     int p = 1;
@@ -1318,44 +1587,33 @@ inline int next_pow2(int v) {
     return p;
 }
 
-template <bool WRITE>
-void spgemm_pass(const rb_csr_s& A, const rb_csr_s& B, const int* bins, const int* bcount,
-                 const std::vector<int>& big_rows_tsize, const DevArray<long long>& toff,
-                 const DevArray<int>& tsize, DevArray<int>& gkeys, DevArray<double>& gsums,
-                 DevArray<int>& glist, int* cnt, const int* crp, int* cci, double* ccv) {
-    const int n = A.n_rows;
-    if (bcount[0]) {
-        size_t sm = (size_t)kW0 * kH0 * (sizeof(double) + 2 * sizeof(int));
-        auto kern = k_spgemm_smem<WRITE, kH0, kW0>;
-        RB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        kern<<<grid_for(bcount[0], kW0), kW0 * 32, sm, stream()>>>(
-            bins, bcount[0], A.rowptr.get(), A.cols.get(), A.vals.get(), B.rowptr.get(),
-            B.cols.get(), B.vals.get(), cnt, crp, cci, ccv);
-        RB_CHECK_LAUNCH();
-    }
-    if (bcount[1]) {
-        size_t sm = (size_t)kW1 * kH1 * (sizeof(double) + 2 * sizeof(int));
-        auto kern = k_spgemm_smem<WRITE, kH1, kW1>;
-        RB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        kern<<<grid_for(bcount[1], kW1), kW1 * 32, sm, stream()>>>(
-            bins + (size_t)n, bcount[1], A.rowptr.get(), A.cols.get(), A.vals.get(),
-            B.rowptr.get(), B.cols.get(), B.vals.get(), cnt, crp, cci, ccv);
-        RB_CHECK_LAUNCH();
-    }
-    if (bcount[2]) {
-        k_spgemm_global<WRITE><<<grid_for((long)bcount[2] * 32, 128), 128, 0, stream()>>>(
-            bins + 2 * (size_t)n, bcount[2], toff.get(), tsize.get(), A.rowptr.get(),
-            A.cols.get(), A.vals.get(), B.rowptr.get(), B.cols.get(), B.vals.get(), gkeys.get(),
-            gsums.get(), glist.get(), cnt, crp, cci, ccv);
-        RB_CHECK_LAUNCH();
-    }
-    (void)big_rows_tsize;
-}
-}  // namespace
-
 namespace {
-constexpr int kK0 = 1024, kKW0 = 16;   // key pass: 16 warps x 1024 x 4 B = 64 KB
-constexpr int kK1 = 8192, kKW1 = 4;    // key pass: 4 warps x 8192 x 4 B = 128 KB
+// One launch of a shared-table kernel over the rows of a list.
+template <int G, int H, int WPB>
+void spgemm_keys_launch(const int* rows, int count, const rb_csr_s& A, const rb_csr_s& B, int* scnt,
+                        int* over, int* over_count) {
+    if (!count) return;
+    constexpr size_t sm = (size_t)WPB * (32 / G) * H * sizeof(int);
+    auto kern = k_spgemm_keys<G, H, WPB>;
+    RB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    kern<<<grid_for(count, WPB * (32 / G)), WPB * 32, sm, stream()>>>(
+        rows, count, A.rowptr.get(), A.cols.get(), B.rowptr.get(), B.cols.get(), scnt, over,
+        over_count);
+    RB_CHECK_LAUNCH();
+}
+
+template <int G, int H, int WPB>
+void spgemm_smem_launch(const int* rows, int count, const rb_csr_s& A, const rb_csr_s& B, int* cnt,
+                        const int* crp, int* cci, double* ccv) {
+    if (!count) return;
+    constexpr size_t sm = (size_t)WPB * (32 / G) * H * (sizeof(double) + sizeof(int));
+    auto kern = k_spgemm_smem<G, H, WPB>;
+    RB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    kern<<<grid_for(count, WPB * (32 / G)), WPB * 32, sm, stream()>>>(
+        rows, count, A.rowptr.get(), A.cols.get(), A.vals.get(), B.rowptr.get(), B.cols.get(),
+        B.vals.get(), cnt, crp, cci, ccv);
+    RB_CHECK_LAUNCH();
+}
 
 // Global tables (one per row of bin 2), sized from a per-row size.
 struct GlobalTables {
@@ -1389,11 +1647,15 @@ GlobalTables global_tables(const int* bins2, int count, const int* size_dev, int
 }  // namespace
 
 // C = A B in two passes: a key-only pass counts each row's distinct
-// columns (4-byte slots, so four times the warps per SM of the numeric
-// pass), then the numeric pass -- binned by that count, so most rows get
+// columns, then the numeric pass -- binned by that count, so most rows get
 // small shared tables -- forms the sums in A's row order, drops
 // |v| <= 1e-16 and writes the survivors sorted; rows that lost entries to
-// the drop are compacted afterwards.
+// the drop are compacted afterwards.  The key pass starts every row in a
+// small table whatever its bound (the sum of its B rows' lengths, several
+// times the distinct columns of a Galerkin product) and repeats the few that
+// overflow in one sized by the bound: sized by the bound from the start, the
+// clearing of 8192 slots a row was most of R (A P)'s count (64^3 27-point
+// setup, all products: counts 2.37 -> 0.76 ms, numeric passes 2.70 -> 1.61).
 rb_csr_s* spgemm(const rb_csr_s& A, const rb_csr_s& B) {
     RB_REQUIRE(A.n_cols == B.n_rows, "spgemm: inner dimensions differ");
     const int n = A.n_rows;
@@ -1402,42 +1664,52 @@ rb_csr_s* spgemm(const rb_csr_s& A, const rb_csr_s& B) {
         RB_CUDA(cudaMemsetAsync(C->rowptr.get(), 0, sizeof(int), stream()));
         return C;
     }
+    // rows of B of at most 8 entries in the mean: 8 lanes a row of C
+    const bool narrow = B.nnz <= 8LL * B.n_rows;
     // 1. structural counts
-    DevArray<int> ub((size_t)n + 1), bins((size_t)3 * n + 3), bcnt(3), scnt((size_t)n + 1);
-    bcnt.zero();
-    k_spgemm_bound<<<grid_for(n, 256), 256, 0, stream()>>>(n, A.rowptr.get(), A.cols.get(),
-                                                          B.rowptr.get(), ub.get(), bins.get(),
-                                                          bcnt.get(), kK0 / 2, kK1 / 2);
-    RB_CHECK_LAUNCH();
-    int hb[3];
-    bcnt.download(hb, 3);
-    RB_CUDA(cudaStreamSynchronize(stream()));
-    if (hb[0]) {
-        const size_t sm = (size_t)kKW0 * kK0 * sizeof(int);
-        auto kern = k_spgemm_keys<kK0, kKW0>;
-        RB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        kern<<<grid_for(hb[0], kKW0), kKW0 * 32, sm, stream()>>>(
-            bins.get(), hb[0], A.rowptr.get(), A.cols.get(), B.rowptr.get(), B.cols.get(),
-            scnt.get());
-        RB_CHECK_LAUNCH();
+    constexpr int kKeysLarge = 8192;
+    DevArray<int> ub((size_t)n + 1), bins((size_t)kBins * n + kBins), bcnt(kBins),
+        scnt((size_t)n + 1), over((size_t)n + 1), over2((size_t)n + 1), nover(2);
+    nover.zero();
+    int* nov = nover.get();
+    if (narrow) spgemm_keys_launch<8, 256, 16>(nullptr, n, A, B, scnt.get(), over.get(), nov);
+    else spgemm_keys_launch<32, 1024, 16>(nullptr, n, A, B, scnt.get(), over.get(), nov);
+    int h_over = read_scalar(nov);
+    const int* left = over.get();
+    if (narrow && h_over) {
+        spgemm_keys_launch<32, 1024, 16>(left, h_over, A, B, scnt.get(), over2.get(), nov + 1);
+        h_over = read_scalar(nov + 1);
+        left = over2.get();
     }
-    if (hb[1]) {
-        const size_t sm = (size_t)kKW1 * kK1 * sizeof(int);
-        auto kern = k_spgemm_keys<kK1, kKW1>;
-        RB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        kern<<<grid_for(hb[1], kKW1), kKW1 * 32, sm, stream()>>>(
-            bins.get() + (size_t)n, hb[1], A.rowptr.get(), A.cols.get(), B.rowptr.get(),
-            B.cols.get(), scnt.get());
+    if (h_over) {
+        // the rest, in tables sized by the bound: those within 8192 keys at a
+        // load of 3/4 in shared memory, the others in global scratch
+        k_spgemm_bound<<<grid_for(n, 256), 256, 0, stream()>>>(n, A.rowptr.get(), A.cols.get(),
+                                                              B.rowptr.get(), ub.get());
         RB_CHECK_LAUNCH();
-    }
-    if (hb[2]) {
-        GlobalTables g = global_tables(bins.get() + 2 * (size_t)n, hb[2], ub.get(), n);
-        DevArray<int> gkeys((size_t)g.total);
-        k_spgemm_keys_global<<<grid_for((long)hb[2] * 32, 128), 128, 0, stream()>>>(
-            bins.get() + 2 * (size_t)n, hb[2], g.toff.get(), g.tsize.get(), A.rowptr.get(),
-            A.cols.get(), B.rowptr.get(), B.cols.get(), gkeys.get(), scnt.get());
-        RB_CHECK_LAUNCH();
+        std::vector<int> rows((size_t)h_over), ubh((size_t)n), small, large;
+        RB_CUDA(cudaMemcpyAsync(rows.data(), left, sizeof(int) * h_over, cudaMemcpyDeviceToHost, stream()));
+        ub.download(ubh.data(), n);
         RB_CUDA(cudaStreamSynchronize(stream()));
+        for (int r : rows) (ubh[r] <= kKeysLarge / 4 * 3 ? small : large).push_back(r);
+        DevArray<int> list((size_t)h_over + 1);
+        list.upload(small.data(), small.size());
+        if (!large.empty())
+            RB_CUDA(cudaMemcpyAsync(list.get() + small.size(), large.data(), sizeof(int) * large.size(),
+                                    cudaMemcpyHostToDevice, stream()));
+        spgemm_keys_launch<32, kKeysLarge, 4>(list.get(), (int)small.size(), A, B, scnt.get(),
+                                              over.get(), nov);
+        if (!large.empty()) {
+            const int* big = list.get() + small.size();
+            GlobalTables g = global_tables(big, (int)large.size(), ub.get(), n);
+            DevArray<int> gkeys((size_t)g.total);
+            k_spgemm_keys_global<<<grid_for((long)large.size() * 32, 128), 128, 0, stream()>>>(
+                big, (int)large.size(), g.toff.get(), g.tsize.get(), A.rowptr.get(),
+                A.cols.get(), B.rowptr.get(), B.cols.get(), gkeys.get(), scnt.get());
+            RB_CHECK_LAUNCH();
+            RB_CUDA(cudaStreamSynchronize(stream()));
+        }
+        RB_CUDA(cudaStreamSynchronize(stream()));   // (list's host copies)
     }
     // 2. capacity layout and numeric pass binned by the structural counts
     DevArray<int> cap((size_t)n + 1);
@@ -1446,23 +1718,35 @@ rb_csr_s* spgemm(const rb_csr_s& A, const rb_csr_s& B) {
     DevArray<int> cols((size_t)std::max<long long>(capacity, 1));
     DevArray<double> vals((size_t)std::max<long long>(capacity, 1));
     bcnt.zero();
-    k_bin_rows<<<grid_for(n, 256), 256, 0, stream()>>>(n, scnt.get(), kH0 / 2, kH1 / 2,
+    // tables at most half full: 128 slots (8 lanes a row when narrow) or 256,
+    // then 512 and 4096, then global scratch
+    const int lim0 = narrow ? 64 : 128;
+    k_bin_rows<<<grid_for(n, 256), 256, 0, stream()>>>(n, scnt.get(), BinLimits{{lim0, 256, 2048}},
                                                        bins.get(), bcnt.get());
     RB_CHECK_LAUNCH();
-    bcnt.download(hb, 3);
+    int hb[kBins];
+    bcnt.download(hb, kBins);
     RB_CUDA(cudaStreamSynchronize(stream()));
-    GlobalTables g = global_tables(bins.get() + 2 * (size_t)n, hb[2], scnt.get(), n);
+    DevArray<int> cnt((size_t)n + 1);
+    const int* b0 = bins.get();
+    const size_t N = (size_t)n;
+    if (narrow) spgemm_smem_launch<8, 128, 8>(b0, hb[0], A, B, cnt.get(), cap.get(), cols.get(), vals.get());
+    else spgemm_smem_launch<32, 256, 8>(b0, hb[0], A, B, cnt.get(), cap.get(), cols.get(), vals.get());
+    spgemm_smem_launch<32, 512, 8>(b0 + N, hb[1], A, B, cnt.get(), cap.get(), cols.get(), vals.get());
+    spgemm_smem_launch<32, 4096, 2>(b0 + 2 * N, hb[2], A, B, cnt.get(), cap.get(), cols.get(), vals.get());
+    GlobalTables g = global_tables(b0 + 3 * N, hb[3], scnt.get(), n);
     DevArray<int> gkeys, glist;
     DevArray<double> gsums;
-    if (hb[2]) {
+    if (hb[3]) {
         gkeys.alloc((size_t)g.total);
         gsums.alloc((size_t)g.total);
         glist.alloc((size_t)g.total);
+        k_spgemm_global<<<grid_for((long)hb[3] * 32, 128), 128, 0, stream()>>>(
+            b0 + 3 * N, hb[3], g.toff.get(), g.tsize.get(), A.rowptr.get(), A.cols.get(),
+            A.vals.get(), B.rowptr.get(), B.cols.get(), B.vals.get(), gkeys.get(), gsums.get(),
+            glist.get(), cnt.get(), cap.get(), cols.get(), vals.get());
+        RB_CHECK_LAUNCH();
     }
-    DevArray<int> cnt((size_t)n + 1);
-    std::vector<int> unused;
-    spgemm_pass<true>(A, B, bins.get(), hb, unused, g.toff, g.tsize, gkeys, gsums, glist,
-                      cnt.get(), cap.get(), cols.get(), vals.get());
     // 3. final layout: the capacity one unless the drop removed entries
     DevArray<int> crp((size_t)n + 1);
     const long long nnz = exclusive_scan(cnt.get(), crp.get(), n);
