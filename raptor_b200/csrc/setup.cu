@@ -760,6 +760,7 @@ struct ExtWarpMem {
     int pos[H];
     int list[CAP];
     double vals[CAP];
+    double fold[32];                        // terms of an ordered sum
 };
 
 __device__ __forceinline__ unsigned ext_hash(int c) { return (unsigned)c * 2654435761u; }
@@ -885,7 +886,7 @@ k_ext_pattern_warp(int n, const int* __restrict__ srp, const int* __restrict__ s
 
 // Rows of 1 .. kExtSmall entries (CAP = kExtSmall) or of more, up to CAP.
 template <int CAP>
-__global__ void __launch_bounds__(kExtWarps * 32)
+__global__ void __launch_bounds__(kExtWarps * 32, 4)
 k_ext_fill_warp(int n, const int* __restrict__ arp, const int* __restrict__ aci,
                 const double* __restrict__ acv, const int* __restrict__ srp,
                 const int* __restrict__ sci, const int* __restrict__ cs,
@@ -969,8 +970,9 @@ k_ext_fill_warp(int n, const int* __restrict__ arp, const int* __restrict__ aci,
                 if (stt != kUnselected) continue;
                 const double sg = (double)__shfl_sync(0xffffffffu, sign, t);
                 // col_sum: the qualifying entries of row col, summed in order
-                // (an entry that does not qualify adds +0, which changes no
-                // sum that starts at +0)
+                // (moved to the front of w.fold and read back by every lane:
+                // passing each of 32 entries round by shuffles kept the
+                // shuffle unit busy for most of the kernel)
                 double col_sum = 0;
                 int id = -1;   // of the first 32 entries, kept for the expansion
                 bool neg = false;
@@ -987,13 +989,13 @@ k_ext_fill_warp(int n, const int* __restrict__ arp, const int* __restrict__ aci,
                         q = ng && f >= 0;
                         if (base == bc) { id = f; neg = ng; }
                     }
-                    const double vq = q ? vk : 0.0;
-                    const int cnt = min(32, ec - base);
-                    for (int u0 = 0; u0 < cnt; u0 += 8) {
-#pragma unroll
-                        for (int u = 0; u < 8; u++)
-                            col_sum = dadd(col_sum, __shfl_sync(0xffffffffu, vq, u0 + u));
-                    }
+                    const unsigned bal = __ballot_sync(0xffffffffu, q);
+                    if (q) w.fold[__popc(bal & ((1u << lane) - 1))] = vk;
+                    __syncwarp();
+                    const int cnt = __popc(bal);
+#pragma unroll 4
+                    for (int u = 0; u < cnt; u++) col_sum = dadd(col_sum, w.fold[u]);
+                    __syncwarp();
                 }
                 if (fabs(col_sum) < kZeroTol) {
                     weak_sum = dadd(weak_sum, valt);

@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
+from tests.test_gpu_parity import assert_csr_equal, oc_tuple, rb_tuple
 
 pytestmark = pytest.mark.gpu
 
@@ -102,5 +103,4 @@ def test_extended_interpolation_with_large_sets(width):
     Ao = O.CSR.from_arrays(n, n, *A.arrays())
     So = O.classical_strength(Ao, 0.25)
     Po = O.interpolation(Ao, So, states, "extended", 0.0)
-    for got, want in zip(P.arrays(), Po.arrays()):
-        np.testing.assert_array_equal(got, want)
+    assert_csr_equal(rb_tuple(P), oc_tuple(Po))
