@@ -60,6 +60,8 @@ float time_launch(F&& fn, const void* warm = nullptr, size_t warm_bytes = 0) {
     return best;
 }
 
+struct SolveCtl;     // state of the stationary solve's device-side loop (hierarchy.cu)
+constexpr int kSolveChunk = 1024;   // iterations one launch of that loop may run
 struct BlockState;   // k right-hand-side buffers and tile shapes (block.cu)
 
 // FP64 result of setup for one level (multilevel/par_level.hpp:15-43).
@@ -147,6 +149,7 @@ struct Hierarchy {
     // Krylov work vectors (finest size) and device scalars
     DevArray<double> kr, kz, kp, kAp, ks, kAs, krs, kph, ksh;
     DevArray<KScal> scal;
+    DevArray<SolveCtl> solve_ctl;
     KScal* host_scal = nullptr;
     PcgCtl* host_ctl = nullptr;   // pinned staging of the device-side loop state
     int gA0 = 0;
