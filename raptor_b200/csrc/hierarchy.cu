@@ -1576,26 +1576,6 @@ void Hierarchy::cycle(double* x, const double* b, bool x_zero) {
 }
 
 // ------------------------------------------------ FP32-form PCG fusions --
-// x += alpha p ; r -= alpha Ap ; rr = r.r, and the FP32 copy of r that the
-// V-cycle takes as its right-hand side (saves the separate conversion pass)
-template <class Fin>
-__global__ void __launch_bounds__(256)
-k_cg_update_f32(long n, double* __restrict__ x, double* __restrict__ r,
-                const double* __restrict__ p, const double* __restrict__ Ap,
-                const KScal* __restrict__ s, float* __restrict__ r32, ReduceSlot rs, Fin fin) {
-    const double alpha = s->alpha;
-    double t = 0.0;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (long)gridDim.x * blockDim.x) {
-        x[i] += p[i] * alpha;
-        const double ri = r[i] + Ap[i] * (-1.0 * alpha);
-        r[i] = ri;
-        r32[i] = (float)ri;
-        t += ri * ri;
-    }
-    block_reduce_finish(t, rs, fin);
-}
-
 // r.z with z the FP32 V-cycle's output, widened to FP64 as it is read: the
 // preconditioned residual is never stored in FP64 (the p update reads the
 // FP32 copy too), which saves 12 of the 24 bytes a row a conversion pass
@@ -1604,11 +1584,7 @@ template <class Fin>
 __global__ void __launch_bounds__(256)
 k_dot_z32(long n, const float* __restrict__ z32, const double* __restrict__ r, ReduceSlot rs,
           Fin fin) {
-    double t = 0.0;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (long)gridDim.x * blockDim.x)
-        t += r[i] * (double)z32[i];
-    block_reduce_finish(t, rs, fin);
+    block_reduce_finish(dot_rows(r, z32, n), rs, fin);
 }
 
 // ------------------------------------------------------------ reductions --
@@ -1886,14 +1862,10 @@ int Hierarchy::pcg(const rb_csr_s& A, double* x, const double* b, double tol, in
         // replacement below keeps the recurrence tied to the FP64 operator.
         outer_apply(A, lowprec, p, Ap, FinPAp{S});
         // x += alpha p ; r -= alpha Ap (or r = b - A x every 8th iteration)
-        if (fp32 && !full_r) {
-            // the update also writes the cycle's FP32 right-hand side
-            k_cg_update_f32<<<rg, 256, 0, stream()>>>(n, x, r, p, Ap, S, lv32[0].b.get(),
-                                                      global_reduce_slot(rg), FinSetRR{S});
-        } else {
-            k_cg_update<<<rg, 256, 0, stream()>>>(n, x, r, p, Ap, S, full_r ? 0 : 1,
-                                                  global_reduce_slot(rg), FinSetRR{S});
-        }
+        // (in the FP32 form the update also writes the cycle's right-hand side)
+        k_cg_update<<<rg, 256, 0, stream()>>>(n, x, r, p, Ap, S, full_r ? 0 : 1,
+                                              fp32 && !full_r ? lv32[0].b.get() : nullptr,
+                                              global_reduce_slot(rg), FinSetRR{S});
         RB_CHECK_LAUNCH();
         if (full_r) {
             true_residual(A, x, b, r);
@@ -1934,9 +1906,9 @@ int Hierarchy::pcg(const rb_csr_s& A, double* x, const double* b, double tol, in
         int pmode = 0;   // p = z already (set above)
         auto iteration = [&](bool full_r, cudaGraphConditionalHandle h, int use_cond) {
             if (fp32)
-                k_cg_p_dev<<<grid_for(n, 256), 256, 0, stream()>>>(n, p, (const float*)lv32[0].x.get(), S);
+                k_cg_p_dev<<<grid_for((n + 1) / 2, 256), 256, 0, stream()>>>(n, p, (const float*)lv32[0].x.get(), S);
             else
-                k_cg_p_dev<<<grid_for(n, 256), 256, 0, stream()>>>(n, p, (const double*)z, S);
+                k_cg_p_dev<<<grid_for((n + 1) / 2, 256), 256, 0, stream()>>>(n, p, (const double*)z, S);
             RB_CHECK_LAUNCH();
             body(full_r);
             k_pcg_step_end<<<1, 32, 0, stream()>>>(S, h, use_cond);
@@ -2020,10 +1992,10 @@ int Hierarchy::pcg(const rb_csr_s& A, double* x, const double* b, double tol, in
         // p = z + beta p  (restart p = z after a full residual)
         const bool restart = (mode == RB_PCG_REFERENCE) && full_r;
         if (fp32)
-            k_cg_p<<<grid_for(n, 256), 256, 0, stream()>>>(n, p, (const float*)lv32[0].x.get(), S,
+            k_cg_p<<<grid_for((n + 1) / 2, 256), 256, 0, stream()>>>(n, p, (const float*)lv32[0].x.get(), S,
                                                            restart ? 1 : 0);
         else
-            k_cg_p<<<grid_for(n, 256), 256, 0, stream()>>>(n, p, (const double*)z, S,
+            k_cg_p<<<grid_for((n + 1) / 2, 256), 256, 0, stream()>>>(n, p, (const double*)z, S,
                                                            restart ? 1 : 0);
         RB_CHECK_LAUNCH();
     }
