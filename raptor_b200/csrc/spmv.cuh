@@ -125,6 +125,10 @@ struct EpiAppend {
     TY* y;
     template <typename A>
     __device__ void operator()(long i, A s, double&) const { y[i] = (TY)((A)y[i] + s); }
+    struct Pre { TY y; };
+    __device__ Pre pre(long i) const { return Pre{y[i]}; }   // (this thread writes y[i] later)
+    template <typename A>
+    __device__ void post(long i, A s, double&, const Pre& p) const { y[i] = (TY)((A)p.y + s); }
 };
 
 // y = x + P xc written to a second buffer (prolongation that also moves the
@@ -135,6 +139,10 @@ struct EpiAddTo {
     TY* y;
     template <typename A>
     __device__ void operator()(long i, A s, double&) const { y[i] = (TY)((A)x0[i] + s); }
+    struct Pre { TY x0; };
+    __device__ Pre pre(long i) const { return Pre{__ldg(x0 + i)}; }
+    template <typename A>
+    __device__ void post(long i, A s, double&, const Pre& p) const { y[i] = (TY)((A)p.x0 + s); }
 };
 
 // Jacobi / L1-Jacobi: xn = xo + dinv (b - A xo); dinv already holds w/d_i.
@@ -273,8 +281,7 @@ struct NoFinish {
 // all of its gathers of x, then the products, so the gathers of a whole
 // batch are in flight together (rows shorter than a batch predicate the
 // rest off).  The products are added in increasing j, the same order as one
-// nonzero at a time.  RB_ROWS_BATCH 0 keeps the older loop (four nonzeros
-// ahead, then the tail one at a time).  Measured on the 192^3 FP32 cycle
+// nonzero at a time.  Measured on the 192^3 FP32 cycle
 // (levels 1-2, G = 8): batches of 4 cut the level-1 residual and sweep from
 // 0.0698 to 0.0661 / 0.0677 ms and the cycle from 0.756 to 0.741 ms; batches
 // of 8 were slower (0.0718 / 0.0885 ms).
@@ -311,107 +318,90 @@ __device__ __forceinline__ Acc row_batched(int j, int e, const CI* __restrict__ 
     return sum;
 }
 
-template <int G, typename TV, typename TX, class Epi>
-__global__ void RB_ROWS_BOUNDS
-k_csr_rows(long n, const int* __restrict__ rp, const int* __restrict__ ci,
-           const TV* __restrict__ cv, const TX* __restrict__ x, Epi epi) {
+// The rows base, base + step, ... below last, RPW = 32 / G rows a warp step,
+// G lanes a row, over 32-bit columns (ci, CI int) or 16-bit offsets from the
+// row's base column (CI unsigned short: column = rbase[row] + ci[j]; 6 bytes
+// a nonzero in FP32 instead of 8).  A step's loads form a chain -- row
+// pointers, then indices and values, then x -- and a warp has little else to
+// do, so the chain is kept short: the next step's row pointers are loaded
+// before this step's entries, and the epilogue's operands (Pre) with them
+// instead of after the row's sum (FP32 cycles: prolongation to 192^3 74 -> 68 us,
+// PCG on 1024^2 12.83 -> 12.13 ms, on 192^3 8.51 -> 8.38; the four FP64 products
+// of a 128^3 27-point matrix 654 -> 618 us).
+template <int G, typename CI, typename TV, typename TX, class Epi>
+__device__ __forceinline__ void rows_walk(long base, long step, long last,
+                                          const int* __restrict__ rp,
+                                          const int* __restrict__ rbase,
+                                          const CI* __restrict__ ci, const TV* __restrict__ cv,
+                                          const TX* __restrict__ x, const Epi& epi) {
     using Acc = AccOf2<TV, TX>;
     constexpr bool SC = ScaledGather<Epi>::value;
-    if constexpr (HasGate<Epi>::value) {
-        if (!epi.open()) return;
-    }
+    constexpr bool I16 = sizeof(CI) == 2;
     const TX* xs = gather_scale_of<Epi, TX>(epi);
-    constexpr int RPW = 32 / G;
     const int lane = threadIdx.x & 31;
     const int sub = lane / G, gl = lane & (G - 1);
-    const long gwarp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
+    auto skip = [&](long b) {
+        if constexpr (HasRowSkip<Epi>::value) return b < last && epi.skip(b);
+        else return false;
+    };
+    int s = 0, e = 0, b0 = 0;
+    auto bounds = [&](long b, bool closed) {
+        s = e = b0 = 0;
+        if (!closed && b + sub < last) {
+            s = __ldg(rp + b + sub);
+            e = __ldg(rp + b + sub + 1);
+            if constexpr (I16) b0 = __ldg(rbase + b + sub);
+        }
+    };
     double red = 0.0;
-    for (long base = gwarp * RPW; base < n; base += nwarps * RPW) {
-        if constexpr (HasRowSkip<Epi>::value) {
-            if (epi.skip(base)) continue;
-        }
+    bool closed = skip(base);
+    bounds(base, closed);
+    for (; base < last; base += step) {
         const long row = base + sub;
-        const bool valid = row < n;
-        int s = 0, e = 0;
-        if (valid) { s = __ldg(rp + row); e = __ldg(rp + row + 1); }
-#if RB_ROWS_BATCH > 0
-        Acc sum = row_batched<G, RB_ROWS_BATCH, Acc, SC>(s + gl, e, ci, cv, x, xs);
-#else
-        static_assert(!SC, "scaled gathers need the batched row loop");
-        Acc sum = 0;
-        int j = s + gl;
-        // four independent index/value loads ahead of their gathers
-        for (; j + 3 * G < e; j += 4 * G) {
-            const int c0 = __ldg(ci + j), c1 = __ldg(ci + j + G);
-            const int c2 = __ldg(ci + j + 2 * G), c3 = __ldg(ci + j + 3 * G);
-            const TV v0 = __ldg(cv + j), v1 = __ldg(cv + j + G);
-            const TV v2 = __ldg(cv + j + 2 * G), v3 = __ldg(cv + j + 3 * G);
-            const TX x0 = __ldg(x + c0), x1 = __ldg(x + c1), x2 = __ldg(x + c2), x3 = __ldg(x + c3);
-            sum += (Acc)v0 * (Acc)x0;
-            sum += (Acc)v1 * (Acc)x1;
-            sum += (Acc)v2 * (Acc)x2;
-            sum += (Acc)v3 * (Acc)x3;
+        const int cs = s, ce = e, cb = b0;
+        const bool shut = closed;
+        closed = skip(base + step);
+        bounds(base + step, closed);
+        if (shut) continue;
+        const bool mine = row < last && gl == 0;
+        if constexpr (HasPre<Epi>::value) {
+            typename Epi::Pre pr{};
+            if (mine) pr = epi.pre(row);
+            const Acc sum = group_sum<G>(row_batched<G, RB_ROWS_BATCH, Acc, SC>(
+                cs + gl, ce, ci, cv, x + cb, SC ? xs + cb : nullptr));
+            if (mine) epi.post(row, sum, red, pr);
+        } else {
+            const Acc sum = group_sum<G>(row_batched<G, RB_ROWS_BATCH, Acc, SC>(
+                cs + gl, ce, ci, cv, x + cb, SC ? xs + cb : nullptr));
+            if (mine) epi(row, sum, red);
         }
-        for (; j < e; j += G) sum += (Acc)__ldg(cv + j) * (Acc)__ldg(x + __ldg(ci + j));
-#endif
-        sum = group_sum<G>(sum);
-        if (valid && gl == 0) epi(row, sum, red);
     }
     (void)red;
 }
 
-// The same row kernel over 16-bit column offsets: column = base[row] +
-// c16[j].  For operators whose rows each span fewer than 65536 columns it
-// reads 2 bytes of index per nonzero instead of 4 (FP32 values: 6 bytes per
-// nonzero instead of 8).
+// The strided schedule: the grid's warps walk the rows together.
+template <int G, typename TV, typename TX, class Epi>
+__global__ void RB_ROWS_BOUNDS
+k_csr_rows(long n, const int* __restrict__ rp, const int* __restrict__ ci,
+           const TV* __restrict__ cv, const TX* __restrict__ x, Epi epi) {
+    if constexpr (HasGate<Epi>::value) {
+        if (!epi.open()) return;
+    }
+    constexpr int RPW = 32 / G;
+    const long gwarp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
+    rows_walk<G>(gwarp * RPW, nwarps * RPW, n, rp, nullptr, ci, cv, x, epi);
+}
+
 template <int G, typename TV, typename TX, class Epi>
 __global__ void RB_ROWS_BOUNDS
 k_csr_rows16(long n, const int* __restrict__ rp, const int* __restrict__ rbase,
              const unsigned short* __restrict__ ci, const TV* __restrict__ cv,
              const TX* __restrict__ x, Epi epi) {
-    using Acc = AccOf2<TV, TX>;
-    constexpr bool SC = ScaledGather<Epi>::value;
-    const TX* xs = gather_scale_of<Epi, TX>(epi);
     constexpr int RPW = 32 / G;
-    const int lane = threadIdx.x & 31;
-    const int sub = lane / G, gl = lane & (G - 1);
     const long gwarp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
-    double red = 0.0;
-    for (long base = gwarp * RPW; base < n; base += nwarps * RPW) {
-        if constexpr (HasRowSkip<Epi>::value) {
-            if (epi.skip(base)) continue;
-        }
-        const long row = base + sub;
-        const bool valid = row < n;
-        int s = 0, e = 0, b0 = 0;
-        if (valid) { s = __ldg(rp + row); e = __ldg(rp + row + 1); b0 = __ldg(rbase + row); }
-        const TX* xb = x + b0;
-#if RB_ROWS_BATCH > 0
-        Acc sum = row_batched<G, RB_ROWS_BATCH, Acc, SC>(s + gl, e, ci, cv, xb,
-                                                         SC ? xs + b0 : nullptr);
-#else
-        static_assert(!SC, "scaled gathers need the batched row loop");
-        Acc sum = 0;
-        int j = s + gl;
-        for (; j + 3 * G < e; j += 4 * G) {
-            const int c0 = __ldg(ci + j), c1 = __ldg(ci + j + G);
-            const int c2 = __ldg(ci + j + 2 * G), c3 = __ldg(ci + j + 3 * G);
-            const TV v0 = __ldg(cv + j), v1 = __ldg(cv + j + G);
-            const TV v2 = __ldg(cv + j + 2 * G), v3 = __ldg(cv + j + 3 * G);
-            const TX x0 = __ldg(xb + c0), x1 = __ldg(xb + c1), x2 = __ldg(xb + c2), x3 = __ldg(xb + c3);
-            sum += (Acc)v0 * (Acc)x0;
-            sum += (Acc)v1 * (Acc)x1;
-            sum += (Acc)v2 * (Acc)x2;
-            sum += (Acc)v3 * (Acc)x3;
-        }
-        for (; j < e; j += G) sum += (Acc)__ldg(cv + j) * (Acc)__ldg(xb + __ldg(ci + j));
-#endif
-        sum = group_sum<G>(sum);
-        if (valid && gl == 0) epi(row, sum, red);
-    }
-    (void)red;
+    rows_walk<G>(gwarp * RPW, nwarps * RPW, n, rp, rbase, ci, cv, x, epi);
 }
 
 // The same row kernels with a blocked schedule: one block of
@@ -424,35 +414,26 @@ k_csr_rows16(long n, const int* __restrict__ rp, const int* __restrict__ rbase,
 constexpr int kRowBlockBlk = 1024;
 constexpr int kRowsBlocked = 64;
 
+// First and one past the last row of this block's share.
+template <int G>
+__device__ __forceinline__ void block_rows(long n, long& first, long& last) {
+    constexpr int RPW = 32 / G;
+    const long per = ((n + gridDim.x - 1) / gridDim.x + RPW - 1) / RPW * RPW;
+    first = (long)blockIdx.x * per;
+    last = first + per < n ? first + per : n;
+}
+
 template <int G, typename TV, typename TX, class Epi>
 __global__ void __launch_bounds__(kRowBlockBlk, 1)
 k_csr_rows_blk(long n, const int* __restrict__ rp, const int* __restrict__ ci,
                const TV* __restrict__ cv, const TX* __restrict__ x, Epi epi) {
-    using Acc = AccOf2<TV, TX>;
-    constexpr bool SC = ScaledGather<Epi>::value;
     if constexpr (HasGate<Epi>::value) {
         if (!epi.open()) return;
     }
-    const TX* xs = gather_scale_of<Epi, TX>(epi);
-    constexpr int RPW = 32 / G;
-    const int lane = threadIdx.x & 31;
-    const int sub = lane / G, gl = lane & (G - 1);
-    const long per = ((n + gridDim.x - 1) / gridDim.x + RPW - 1) / RPW * RPW;
-    const long first = (long)blockIdx.x * per;
-    const long last = first + per < n ? first + per : n;
-    const int warp = threadIdx.x >> 5;
-    const int nw = blockDim.x >> 5;
-    double red = 0.0;
-    for (long base = first + (long)warp * RPW; base < last; base += (long)nw * RPW) {
-        const long row = base + sub;
-        const bool valid = row < last;
-        int s = 0, e = 0;
-        if (valid) { s = __ldg(rp + row); e = __ldg(rp + row + 1); }
-        Acc sum = row_batched<G, RB_ROWS_BATCH, Acc, SC>(s + gl, e, ci, cv, x, xs);
-        sum = group_sum<G>(sum);
-        if (valid && gl == 0) epi(row, sum, red);
-    }
-    (void)red;
+    long first, last;
+    block_rows<G>(n, first, last);
+    rows_walk<G>(first + (long)(threadIdx.x >> 5) * (32 / G), (long)(blockDim.x >> 5) * (32 / G),
+                 last, rp, nullptr, ci, cv, x, epi);
 }
 
 template <int G, typename TV, typename TX, class Epi>
@@ -460,29 +441,10 @@ __global__ void __launch_bounds__(kRowBlockBlk, 1)
 k_csr_rows16_blk(long n, const int* __restrict__ rp, const int* __restrict__ rbase,
                  const unsigned short* __restrict__ ci, const TV* __restrict__ cv,
                  const TX* __restrict__ x, Epi epi) {
-    using Acc = AccOf2<TV, TX>;
-    constexpr bool SC = ScaledGather<Epi>::value;
-    const TX* xs = gather_scale_of<Epi, TX>(epi);
-    constexpr int RPW = 32 / G;
-    const int lane = threadIdx.x & 31;
-    const int sub = lane / G, gl = lane & (G - 1);
-    const long per = ((n + gridDim.x - 1) / gridDim.x + RPW - 1) / RPW * RPW;
-    const long first = (long)blockIdx.x * per;
-    const long last = first + per < n ? first + per : n;
-    const int warp = threadIdx.x >> 5;
-    const int nw = blockDim.x >> 5;
-    double red = 0.0;
-    for (long base = first + (long)warp * RPW; base < last; base += (long)nw * RPW) {
-        const long row = base + sub;
-        const bool valid = row < last;
-        int s = 0, e = 0, b0 = 0;
-        if (valid) { s = __ldg(rp + row); e = __ldg(rp + row + 1); b0 = __ldg(rbase + row); }
-        Acc sum = row_batched<G, RB_ROWS_BATCH, Acc, SC>(s + gl, e, ci, cv, x + b0,
-                                                         SC ? xs + b0 : nullptr);
-        sum = group_sum<G>(sum);
-        if (valid && gl == 0) epi(row, sum, red);
-    }
-    (void)red;
+    long first, last;
+    block_rows<G>(n, first, last);
+    rows_walk<G>(first + (long)(threadIdx.x >> 5) * (32 / G), (long)(blockDim.x >> 5) * (32 / G),
+                 last, rp, rbase, ci, cv, x, epi);
 }
 
 template <int G, typename TV, class Fin>
@@ -501,24 +463,7 @@ k_csr_rows_dot(long n, const int* __restrict__ rp, const int* __restrict__ ci,
         const bool valid = row < n;
         int s = 0, e = 0;
         if (valid) { s = __ldg(rp + row); e = __ldg(rp + row + 1); }
-#if RB_ROWS_BATCH > 0
         double sum = row_batched<G, RB_ROWS_BATCH, double>(s + gl, e, ci, cv, x);
-#else
-        double sum = 0;
-        int j = s + gl;
-        for (; j + 3 * G < e; j += 4 * G) {
-            const int c0 = __ldg(ci + j), c1 = __ldg(ci + j + G);
-            const int c2 = __ldg(ci + j + 2 * G), c3 = __ldg(ci + j + 3 * G);
-            const TV v0 = __ldg(cv + j), v1 = __ldg(cv + j + G);
-            const TV v2 = __ldg(cv + j + 2 * G), v3 = __ldg(cv + j + 3 * G);
-            const double x0 = __ldg(x + c0), x1 = __ldg(x + c1), x2 = __ldg(x + c2), x3 = __ldg(x + c3);
-            sum += (double)v0 * x0;
-            sum += (double)v1 * x1;
-            sum += (double)v2 * x2;
-            sum += (double)v3 * x3;
-        }
-        for (; j < e; j += G) sum += (double)__ldg(cv + j) * __ldg(x + __ldg(ci + j));
-#endif
         sum = group_sum<G>(sum);
         if (valid && gl == 0) epi(row, sum, red);
     }
