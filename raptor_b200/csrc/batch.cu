@@ -20,6 +20,7 @@
 #include <string>
 
 #include "blas1.cuh"
+#include "dense_bottom.cuh"
 #include "hierarchy.cuh"
 
 namespace rb {
@@ -98,25 +99,22 @@ __global__ void k_lu_solve_batch(const int* __restrict__ row0, const int* __rest
     for (int i = threadIdx.x; i < n; i += blockDim.x) x[r0 + i] = (T)y[i];
 }
 
-// x = inv b for each listed system's coarsest level (one CTA per system;
-// inverses column-major)
+// x = B b for each listed system's bottom level (its coarsest, or the level
+// its cycle is cut at): matrix sys at doff, row length dense_ld, FP64; a warp
+// a row, blockIdx.y the system.
 template <typename T>
-__global__ void k_coarse_mv_batch(const int* __restrict__ row0, const int* __restrict__ nrow,
-                                  const long long* __restrict__ ioff, const double* __restrict__ inv_all,
-                                  const T* __restrict__ b, T* __restrict__ x,
-                                  const int* __restrict__ sys, const int* __restrict__ active) {
-    if (active && !active[sys[blockIdx.x]]) return;
-    extern __shared__ double bs[];
-    const int n = nrow[blockIdx.x];
-    const long r0 = row0[blockIdx.x];
-    const double* inv = inv_all + ioff[blockIdx.x];
-    for (int i = threadIdx.x; i < n; i += blockDim.x) bs[i] = (double)b[r0 + i];
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        double s = 0.0;
-        for (int j = 0; j < n; j++) s += inv[(size_t)j * n + i] * bs[j];
-        x[r0 + i] = (T)s;
-    }
+__global__ void __launch_bounds__(128)
+k_dense_mv_batch(const int* __restrict__ row0, const int* __restrict__ nrow,
+                 const long long* __restrict__ doff, const double* __restrict__ B_all,
+                 const T* __restrict__ b, T* __restrict__ x, const int* __restrict__ sys,
+                 const int* __restrict__ active) {
+    const int n = nrow[blockIdx.y];
+    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (row >= n || (active && !active[sys[blockIdx.y]])) return;
+    const int ld = (n + 1) & ~1;
+    const long r0 = row0[blockIdx.y];
+    const double s = dense_row(n, ld, B_all + doff[blockIdx.y] + (size_t)row * ld, b + r0);
+    if ((threadIdx.x & 31) == 0) x[r0 + row] = (T)s;
 }
 
 // Segmented dot: one CTA per chunk writes its partial, and the last CTA to
@@ -365,15 +363,20 @@ struct Batch {
     int n_sys = 0;
     rb_amg_opts opts{};
     std::vector<int> depth;                       // levels of each system
+    std::vector<int> cut;                         // levels kept: the last is solved by a dense matrix
+    int max_depth = 0;
     std::vector<std::vector<long long>> off;      // off[l][s], n_sys + 1 entries
     Hierarchy cat;                                // packed levels
     // coarsest-level LUs
-    DevArray<double> lu, inv;   // inv: coarse inverses when every coarsest level is small
+    DevArray<double> lu;
+    // the dense matrices of the levels the systems' cycles end at, when every
+    // coarsest level is small (else the LUs above solve those)
+    DevArray<double> dense;
     DevArray<int> piv;
     struct CoarseTab {
         int count = 0, max_n = 0;
         DevArray<int> row0, n, pivo, sys;
-        DevArray<long long> luo;
+        DevArray<long long> luo, doff;
     };
     std::vector<CoarseTab> coarse;
     // outer CG
@@ -434,9 +437,9 @@ struct Batch {
         CoarseTab& t = coarse[l];
         if (!t.count) return;
         const int* act = gating ? S.active : nullptr;
-        if (inv.get())
-            k_coarse_mv_batch<T><<<t.count, 256, sizeof(double) * std::max(t.max_n, 1), stream()>>>(
-                t.row0.get(), t.n.get(), t.luo.get(), inv.get(), b, x, t.sys.get(), act);
+        if (dense.get())
+            k_dense_mv_batch<T><<<dim3((t.max_n + 3) / 4, t.count), 128, 0, stream()>>>(
+                t.row0.get(), t.n.get(), t.doff.get(), dense.get(), b, x, t.sys.get(), act);
         else
             k_lu_solve_batch<T><<<t.count, 256, sizeof(double) * std::max(t.max_n, 1), stream()>>>(
                 t.row0.get(), t.n.get(), t.luo.get(), t.pivo.get(), lu.get(), piv.get(), b, x,
@@ -445,6 +448,7 @@ struct Batch {
     }
 
     void setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o);
+    void choose_cut(const std::vector<std::unique_ptr<Hierarchy>>& sys, std::vector<long long>& doff);
     template <bool Gt, typename T>
     void cycle_level(std::vector<Level<T>>& lv, int l, T* x, const T* b, bool x_zero);
     void cycle64(double* x, const double* b);
@@ -453,6 +457,53 @@ struct Batch {
                         double* relres, const std::vector<double>& bnorm,
                         const std::function<void()>& restart);
 };
+
+// Where each system's cycle ends.  With the dense bottom (dense_bottom.cuh)
+// a system keeps its levels down to the first one, above the coarsest, of at
+// most kBatchCut rows, halved until the matrices of all systems fit
+// kBatchDenseBytes (an iteration reads them all: at that size about as long
+// as the launches of one packed level take); otherwise, and for a system
+// without such a level, down to its coarsest.  16 systems of 64^2 to 320^2
+// rows: three packed levels fewer, PCG 10.4 -> 9.2 ms.  doff: the matrices' offsets
+// (FP64, rows padded to 16 bytes); empty when a coarsest level is too large
+// for an inverse.
+constexpr int kBatchCut = 1024;
+constexpr long long kBatchDenseBytes = 32LL << 20;
+
+void Batch::choose_cut(const std::vector<std::unique_ptr<Hierarchy>>& sys, std::vector<long long>& doff) {
+    const int n = n_sys;
+    cut = depth;
+    doff.clear();
+    for (int s = 0; s < n; s++)
+        if (sys[s]->master[depth[s] - 1].A->n_rows > kCoarseInvMax) return;
+    auto total = [&](const std::vector<int>& c, std::vector<long long>* at) {
+        long long t = 0;
+        for (int s = 0; s < n; s++) {
+            const int m = sys[s]->master[c[s] - 1].A->n_rows;
+            if (at) (*at)[s] = t;
+            t += (long long)m * dense_ld<double>(m);
+        }
+        if (at) (*at)[n] = t;
+        return t * (long long)sizeof(double);
+    };
+    if (opts.fuse_coarse == 1 && dense_bottom_applies(opts)) {
+        for (int cap = kBatchCut; cap >= 64; cap /= 2) {
+            std::vector<int> c = depth;
+            for (int s = 0; s < n; s++)
+                for (int l = depth[s] - 2; l >= 1; l--) {
+                    const int m = sys[s]->master[l].A->n_rows;
+                    if (m > cap || m == 0 || sys[s]->master[depth[s] - 1].A->n_rows == 0) break;
+                    c[s] = l + 1;
+                }
+            if (total(c, nullptr) <= kBatchDenseBytes) {
+                cut = c;
+                break;
+            }
+        }
+    }
+    doff.assign((size_t)n + 1, 0);
+    total(cut, &doff);
+}
 
 void Batch::setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o) {
     RB_REQUIRE(n >= 1 && n <= 65535, "batch: the number of systems must be in 1..65535");
@@ -470,11 +521,15 @@ void Batch::setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o) {
         depth[s] = sys[s]->num_levels();
         Lmax = std::max(Lmax, depth[s]);
     }
+    max_depth = Lmax;
+    std::vector<long long> doff;
+    choose_cut(sys, doff);
+    Lmax = *std::max_element(cut.begin(), cut.end());
     // row offsets per level (absent systems have no rows)
     off.assign(Lmax, std::vector<long long>(n + 1, 0));
     for (int l = 0; l < Lmax; l++)
         for (int s = 0; s < n; s++)
-            off[l][s + 1] = off[l][s] + (l < depth[s] ? sys[s]->master[l].A->n_rows : 0);
+            off[l][s + 1] = off[l][s] + (l < cut[s] ? sys[s]->master[l].A->n_rows : 0);
     RB_REQUIRE(off[0][n] <= INT_MAX, "batch: more than 2^31-1 rows in total");
     // pack A_l and P_l block-diagonally
     cat.opts = o;
@@ -484,9 +539,9 @@ void Batch::setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o) {
     for (int l = 0; l < Lmax; l++) {
         long long nnzA = 0, nnzP = 0;
         for (int s = 0; s < n; s++) {
-            if (l >= depth[s]) continue;
+            if (l >= cut[s]) continue;
             nnzA += sys[s]->master[l].A->nnz;
-            if (l < depth[s] - 1) nnzP += sys[s]->master[l].P->nnz;
+            if (l < cut[s] - 1) nnzP += sys[s]->master[l].P->nnz;
         }
         const int rows = (int)off[l][n];
         rb_csr_s* A = new_csr(rows, rows, nnzA);
@@ -498,7 +553,7 @@ void Batch::setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o) {
         }
         long long za = 0, zp = 0;
         for (int s = 0; s < n; s++) {
-            if (l >= depth[s]) continue;
+            if (l >= cut[s]) continue;
             const rb_csr_s& As = *sys[s]->master[l].A;
             const int ns = As.n_rows;
             if (ns)
@@ -508,7 +563,7 @@ void Batch::setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o) {
             RB_CHECK_LAUNCH();
             za += As.nnz;
             if (P) {
-                if (l < depth[s] - 1) {
+                if (l < cut[s] - 1) {
                     const rb_csr_s& Ps = *sys[s]->master[l].P;
                     k_pack_rows<<<grid_for(ns, 128), 128, 0, stream()>>>(
                         ns, Ps.rowptr.get(), Ps.cols.get(), Ps.vals.get(), off[l][s], zp,
@@ -516,7 +571,7 @@ void Batch::setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o) {
                     RB_CHECK_LAUNCH();
                     zp += Ps.nnz;
                 } else if (ns) {
-                    // coarsest at l: empty rows of P
+                    // ends at l: empty rows of P
                     k_fill_rowptr<<<grid_for(ns, 128), 128, 0, stream()>>>(ns, off[l][s], (int)zp,
                                                                            P->rowptr.get());
                     RB_CHECK_LAUNCH();
@@ -535,7 +590,8 @@ void Batch::setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o) {
         }
         RB_CUDA(cudaStreamSynchronize(stream()));
     }
-    // coarsest-level LUs (A_c^T, as the standalone hierarchy factors it)
+    // coarsest-level LUs (A_c^T, as the standalone hierarchy factors it), and
+    // the dense matrices formed from their inverses
     std::vector<long long> luo(n), pivo(n);
     long long lu_tot = 0, piv_tot = 0;
     for (int s = 0; s < n; s++) {
@@ -561,16 +617,22 @@ void Batch::setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o) {
         k_lu_factor<<<1, 256, 0, stream()>>>(nc, lu.get() + luo[s], piv.get() + pivo[s], info.get());
         RB_CHECK_LAUNCH();
     }
-    int nc_max = 0;
-    for (int s = 0; s < n; s++) nc_max = std::max(nc_max, sys[s]->master[depth[s] - 1].A->n_rows);
-    if (nc_max <= kCoarseInvMax) {
-        inv.alloc((size_t)std::max(lu_tot, 1LL));
+    dense.release();
+    if (!doff.empty()) {
+        dense.alloc((size_t)std::max(doff[n], 1LL));
         for (int s = 0; s < n; s++) {
-            const int nc = sys[s]->master[depth[s] - 1].A->n_rows;
-            if (!nc) continue;
+            const std::vector<MasterLevel>& M = sys[s]->master;
+            const int nc = M[depth[s] - 1].A->n_rows, nd = M[cut[s] - 1].A->n_rows;
+            if (!nc || !nd) continue;
+            DevArray<double> inv((size_t)nc * nc), B;
             k_lu_invert<<<1, 256, sizeof(double) * nc, stream()>>>(nc, lu.get() + luo[s],
-                                                                  piv.get() + pivo[s],
-                                                                  inv.get() + luo[s]);
+                                                                  piv.get() + pivo[s], inv.get());
+            RB_CHECK_LAUNCH();
+            if (o.precision == RB_PREC_FP32) form_dense_bottom<float>(M, o, cut[s] - 1, inv.get(), nullptr, B);
+            else form_dense_bottom<double>(M, o, cut[s] - 1, inv.get(), nullptr, B);
+            const int ld = dense_ld<double>(nd);
+            k_dense_store<double><<<dim3((ld + 255) / 256, nd), 256, 0, stream()>>>(nd, ld, B.get(),
+                                                                                    dense.get() + doff[s]);
             RB_CHECK_LAUNCH();
         }
     }
@@ -578,16 +640,17 @@ void Batch::setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o) {
     coarse.resize(Lmax);
     for (int l = 0; l < Lmax; l++) {
         std::vector<int> r0, nr, pv, sy;
-        std::vector<long long> lo;
+        std::vector<long long> lo, dof;
         int mx = 0;
         for (int s = 0; s < n; s++) {
-            if (depth[s] - 1 != l) continue;
+            if (cut[s] - 1 != l) continue;
             const int nc = (int)(off[l][s + 1] - off[l][s]);
             if (!nc) continue;
             sy.push_back(s);
             r0.push_back((int)off[l][s]);
             nr.push_back(nc);
             lo.push_back(luo[s]);
+            dof.push_back(doff.empty() ? 0 : doff[s]);
             pv.push_back((int)pivo[s]);
             mx = std::max(mx, nc);
         }
@@ -598,6 +661,7 @@ void Batch::setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o) {
             t.row0.alloc(t.count); t.row0.upload(r0.data(), t.count);
             t.n.alloc(t.count); t.n.upload(nr.data(), t.count);
             t.luo.alloc(t.count); t.luo.upload(lo.data(), t.count);
+            t.doff.alloc(t.count); t.doff.upload(dof.data(), t.count);
             t.pivo.alloc(t.count); t.pivo.upload(pv.data(), t.count);
             t.sys.alloc(t.count); t.sys.upload(sy.data(), t.count);
         }
@@ -1004,7 +1068,7 @@ void batch_destroy(rb_batch_s* B) { delete B; }
 int batch_num_systems(const rb_batch_s* B) { return B->b.n_sys; }
 long long batch_offset(const rb_batch_s* B, int s) { return B->b.off[0][s]; }
 int batch_levels(const rb_batch_s* B, int s) { return B->b.depth[s]; }
-int batch_packed_levels(const rb_batch_s* B) { return (int)B->b.off.size(); }
+int batch_packed_levels(const rb_batch_s* B) { return B->b.max_depth; }
 void batch_cycle(rb_batch_s* B, double* x, const double* b) {
     Batch& T = B->b;
     char key[96];

@@ -34,25 +34,31 @@ inline int dense_ld(int n) {
     return (n + v - 1) / v * v;
 }
 
-// x = B b: one warp a row, 16 bytes a lane and step.  Rows are padded with
-// zeros to ld, and b is read only below n.
-template <typename T>
-__global__ void __launch_bounds__(128)
-k_dense_mv(int n, int ld, const T* __restrict__ B, const T* __restrict__ b, T* __restrict__ x) {
-    constexpr int V = 16 / sizeof(T);
-    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (row >= n) return;
-    const T* r = B + (size_t)row * ld;
+// Row `row` of B b for one warp: 16 bytes a lane and step, rows padded with
+// zeros to ld, b read only below n; every lane gets the sum.
+template <typename TM, typename T>
+__device__ __forceinline__ double dense_row(int n, int ld, const TM* __restrict__ r,
+                                            const T* __restrict__ b) {
+    constexpr int V = 16 / sizeof(TM);
     double s = 0.0;
 #pragma unroll 4
-    for (int j = lane * V; j < ld; j += 32 * V) {
-        T a[V];
+    for (int j = (threadIdx.x & 31) * V; j < ld; j += 32 * V) {
+        TM a[V];
         *reinterpret_cast<uint4*>(a) = __ldg(reinterpret_cast<const uint4*>(r + j));
 #pragma unroll
         for (int v = 0; v < V; v++) s += (double)a[v] * (j + v < n ? (double)__ldg(b + j + v) : 0.0);
     }
-    s = warp_sum(s);
-    if (lane == 0) x[row] = (T)s;
+    return warp_sum(s);
+}
+
+// x = B b, one warp a row
+template <typename T>
+__global__ void __launch_bounds__(128)
+k_dense_mv(int n, int ld, const T* __restrict__ B, const T* __restrict__ b, T* __restrict__ x) {
+    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (row >= n) return;
+    const double s = dense_row(n, ld, B + (size_t)row * ld, b);
+    if ((threadIdx.x & 31) == 0) x[row] = (T)s;
 }
 
 // ------------------------------------------------------- forming B (FP64) --

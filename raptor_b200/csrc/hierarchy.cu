@@ -971,11 +971,7 @@ void Hierarchy::build_dense(std::vector<Level<T>>& lv, DevArray<T>& B) {
     dense_from = -1;
     B.release();
     const int L = (int)lv.size();
-    const int rt = opts.relax_type;
-    const bool none = rt == RB_RELAX_JACOBI && opts.jacobi_compat;
-    const bool jac = (rt == RB_RELAX_JACOBI || rt == RB_RELAX_L1JACOBI) &&
-                     (opts.num_smooth_sweeps == 1 || none);
-    if (opts.fuse_coarse != 1 || !jac || L < 3 || !cinv.get()) return;
+    if (opts.fuse_coarse != 1 || !dense_bottom_applies(opts) || L < 3 || !cinv.get()) return;
     int f = -1;
     for (int l = L - 2; l >= 1; l--) {
         const size_t n = (size_t)lv[l].n;
@@ -983,17 +979,49 @@ void Hierarchy::build_dense(std::vector<Level<T>>& lv, DevArray<T>& B) {
         f = l;
     }
     if (f < 0) return;
+    std::vector<const T*> dinv((size_t)L, nullptr);
+    for (int l = f; l < L - 1; l++) dinv[l] = lv[l].dinv.get();
+    DevArray<double> Bf;
+    form_dense_bottom<T>(master, opts, f, cinv.get(), dinv.data(), Bf);
+    const int n = lv[f].n;
+    dense_ld_ = dense_ld<T>(n);
+    B.alloc((size_t)n * dense_ld_);
+    k_dense_store<T><<<dim3((dense_ld_ + 255) / 256, n), 256, 0, stream()>>>(n, dense_ld_, Bf.get(), B.get());
+    RB_CHECK_LAUNCH();
+    dense_from = f;
+}
+
+bool dense_bottom_applies(const rb_amg_opts& o) {
+    const int rt = o.relax_type;
+    return (rt == RB_RELAX_JACOBI || rt == RB_RELAX_L1JACOBI) &&
+           (o.num_smooth_sweeps == 1 || (rt == RB_RELAX_JACOBI && o.jacobi_compat));
+}
+
+template <typename T>
+void form_dense_bottom(const std::vector<MasterLevel>& master, const rb_amg_opts& o, int f,
+                       const double* cinv, const T* const* dinv, DevArray<double>& B) {
+    const int L = (int)master.size();
+    const bool none = o.relax_type == RB_RELAX_JACOBI && o.jacobi_compat;
+    const int coarse_n = master[L - 1].A->n_rows;
     auto cols = [](int m) { return (unsigned)((m + 255) / 256); };
     auto sp = [](const rb_csr_s& M) { return std::make_tuple(M.rowptr.get(), M.cols.get(), M.vals.get()); };
     DevArray<double> Bc((size_t)coarse_n * coarse_n);
-    k_dense_from_inverse<<<dim3(cols(coarse_n), coarse_n), 256, 0, stream()>>>(coarse_n, cinv.get(), Bc.get());
+    k_dense_from_inverse<<<dim3(cols(coarse_n), coarse_n), 256, 0, stream()>>>(coarse_n, cinv, Bc.get());
     RB_CHECK_LAUNCH();
     for (int l = L - 2; l >= f; l--) {
-        const int n = lv[l].n, nc = lv[l + 1].n;
-        const T* d = lv[l].dinv.get();
+        const int n = master[l].A->n_rows, nc = master[l + 1].A->n_rows;
         const auto [arp, aci, acv] = sp(*master[l].A);
         const auto [prp, pci, pcv] = sp(*master[l].P);
         const auto [rrp, rci, rcv] = sp(*master[l].R);
+        DevArray<T> own;
+        const T* d = dinv ? dinv[l] : nullptr;
+        if (!d) {
+            own.alloc((size_t)n);
+            k_diag_inv<T><<<grid_for(n, 256), 256, 0, stream()>>>(
+                n, arp, aci, acv, o.relax_weight, o.relax_type == RB_RELAX_L1JACOBI ? 1 : 0, own.get());
+            RB_CHECK_LAUNCH();
+            d = own.get();
+        }
         const size_t nn = (size_t)n * n, cn = (size_t)nc * n;
         DevArray<double> W(nn), Tm(cn), E(cn), Bl(nn);
         if (none) {
@@ -1018,13 +1046,12 @@ void Hierarchy::build_dense(std::vector<Level<T>>& lv, DevArray<T>& B) {
         RB_CHECK_LAUNCH();
         Bc = std::move(Bl);
     }
-    const int n = lv[f].n;
-    dense_ld_ = dense_ld<T>(n);
-    B.alloc((size_t)n * dense_ld_);
-    k_dense_store<T><<<dim3(cols(dense_ld_), n), 256, 0, stream()>>>(n, dense_ld_, Bc.get(), B.get());
-    RB_CHECK_LAUNCH();
-    dense_from = f;
+    B = std::move(Bc);
 }
+template void form_dense_bottom<float>(const std::vector<MasterLevel>&, const rb_amg_opts&, int,
+                                       const double*, const float* const*, DevArray<double>&);
+template void form_dense_bottom<double>(const std::vector<MasterLevel>&, const rb_amg_opts&, int,
+                                        const double*, const double* const*, DevArray<double>&);
 
 Hierarchy::~Hierarchy() {
     release_graphs();

@@ -137,6 +137,16 @@ struct Level {
     }
 };
 
+// Whether the bottom of a cycle with these options can be one dense product
+// (dense_bottom.cuh): one Jacobi-type sweep, or the reference's no-op Jacobi.
+bool dense_bottom_applies(const rb_amg_opts& o);
+// B (n_f x n_f, row-major, FP64) of the cycle from level f < L - 1 down, from
+// the coarsest matrix's inverse (column-major).  dinv: the levels' scaled
+// inverse diagonals; NULL: formed from the options in the precision T.
+template <typename T>
+void form_dense_bottom(const std::vector<MasterLevel>& master, const rb_amg_opts& o, int f,
+                       const double* cinv, const T* const* dinv, DevArray<double>& B);
+
 struct Hierarchy {
     rb_amg_opts opts{};
     std::vector<MasterLevel> master;

@@ -1,0 +1,56 @@
+"""The batch whose cycles end in a dense matrix (the level each system is cut
+at is chosen by size, fewer rows when the matrices of all systems would not
+fit) against the batch without it (fuse_coarse = 0) and against standalone
+cycles; the reported levels are those of the whole hierarchies."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+rb = pytest.importorskip("raptor_b200")
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _device():
+    rb.init(0)
+
+
+def make(prec, fuse, relax, compat=0):
+    ml = rb.ParRugeStubenSolver(0.25, rb.PMIS, rb.ModClassical, rb.Classical, relax)
+    ml.precision, ml.fuse_coarse, ml.jacobi_compat = prec, fuse, compat
+    return ml
+
+
+# sides 5 and 7: no coarse level at all, and none above the coarsest; 40 systems
+# of 60 x 60 and more: the cut falls to 512 and 256 rows
+SETS = {"mixed": [5, 7, 13, 40, 90], "one": [64], "many": [60, 64, 68, 72] * 10}
+
+
+@pytest.mark.parametrize("prec", [rb.FP64, rb.FP32], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("sides", sorted(SETS))
+@pytest.mark.parametrize("relax,compat", [(rb.L1Jacobi, 0), (rb.Jacobi, 1), (rb.SOR, 0)],
+                         ids=["l1_jacobi", "jacobi_noop", "sor"])
+def test_batch_cycle_with_and_without_the_cut(sides, prec, relax, compat):
+    mats = [rb.par_stencil_grid(rb.diffusion_stencil_2d(0.05, 0.3 + 0.01 * i), [m, m])
+            for i, m in enumerate(SETS[sides])]
+    got, levels = [], []
+    for fuse in (0, 1):
+        B = rb.Batch(mats, make(prec, fuse, relax, compat))
+        b = rb.ParVector(B.total_rows, values=np.random.default_rng(3).uniform(-1, 1, B.total_rows))
+        x = rb.ParVector(B.total_rows)
+        B.cycle(x, b)
+        got.append(x.numpy())
+        levels.append(list(B.levels))
+    assert levels[0] == levels[1]
+    tol = 1e-11 if prec == rb.FP64 else 1e-4
+    for s, m in enumerate(SETS[sides]):
+        lo, hi = B.offsets[s], B.offsets[s + 1]
+        ref = got[0][lo:hi]
+        assert np.linalg.norm(got[1][lo:hi] - ref) <= tol * np.linalg.norm(ref), (s, m)
+    ml = make(prec, 1, relax, compat)
+    ml.setup(mats[-1])
+    lo, hi = B.offsets[-2], B.offsets[-1]
+    y = rb.ParVector(int(hi - lo))
+    ml.cycle(y, rb.ParVector(int(hi - lo), values=b.numpy()[lo:hi]))
+    assert np.linalg.norm(got[1][lo:hi] - y.numpy()) <= tol * np.linalg.norm(y.numpy())
+    assert ml.num_levels == levels[1][-1]
