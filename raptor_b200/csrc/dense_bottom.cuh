@@ -61,6 +61,34 @@ k_dense_mv(int n, int ld, const T* __restrict__ B, const T* __restrict__ b, T* _
     if ((threadIdx.x & 31) == 0) x[row] = (T)s;
 }
 
+// X = B b for k interleaved columns (entry (j, c) at j k + c): one warp a row
+// and kDenseCols of its columns (blockIdx.y), the row of B read once for them.
+constexpr int kDenseCols = 8;
+template <typename T>
+__global__ void __launch_bounds__(128)
+k_dense_mm(int n, int ld, const T* __restrict__ B, int k, const T* __restrict__ b,
+           T* __restrict__ x) {
+    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const int c0 = blockIdx.y * kDenseCols;
+    if (row >= n) return;
+    const T* r = B + (size_t)row * ld;
+    double s[kDenseCols] = {};
+#pragma unroll 2
+    for (int j = lane; j < n; j += 32) {
+        const double a = (double)__ldg(r + j);
+        T v[kDenseCols];
+#pragma unroll
+        for (int c = 0; c < kDenseCols; c++) v[c] = c0 + c < k ? __ldg(b + (size_t)j * k + c0 + c) : T(0);
+#pragma unroll
+        for (int c = 0; c < kDenseCols; c++) s[c] += a * (double)v[c];
+    }
+#pragma unroll
+    for (int c = 0; c < kDenseCols; c++) {
+        const double t = warp_sum(s[c]);
+        if (lane == 0 && c0 + c < k) x[(size_t)row * k + c0 + c] = (T)t;
+    }
+}
+
 // ------------------------------------------------------- forming B (FP64) --
 // out (n x m, row-major) = the transpose of a column-major n x n matrix
 static __global__ void k_dense_from_inverse(int n, const double* __restrict__ inv, double* out) {

@@ -47,6 +47,8 @@ def test_batch_cycle_with_and_without_the_cut(sides, prec, relax, compat):
         lo, hi = B.offsets[s], B.offsets[s + 1]
         ref = got[0][lo:hi]
         assert np.linalg.norm(got[1][lo:hi] - ref) <= tol * np.linalg.norm(ref), (s, m)
+    if relax == rb.SOR:
+        return   # the batch's rows are coloured as one matrix, not system by system
     ml = make(prec, 1, relax, compat)
     ml.setup(mats[-1])
     lo, hi = B.offsets[-2], B.offsets[-1]
