@@ -450,7 +450,8 @@ struct Batch {
     void setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o);
     void choose_cut(const std::vector<std::unique_ptr<Hierarchy>>& sys, std::vector<long long>& doff);
     template <bool Gt, typename T>
-    void cycle_level(std::vector<Level<T>>& lv, int l, T* x, const T* b, bool x_zero);
+    void cycle_level(std::vector<Level<T>>& lv, int l, T* x, const T* b, bool x_zero,
+                     bool swept = false);
     void cycle64(double* x, const double* b);
     int pcg(double* x, const double* b, double tol, int max_iter, int* iters, double* relres);
     int pcg_device_loop(double* x, const double* b, double tol, int max_iter, int* iters,
@@ -749,8 +750,9 @@ void Batch::setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o) {
 // systems whose coarsest level is l.  Gt: the rows of systems that have
 // stopped are passed over (the row gates; Jacobi-type smoothing only, the
 // multicolour sweeps run every row).
+// swept: x holds the first sweep's result already (EpiStoreScale).
 template <bool Gt, typename T>
-void Batch::cycle_level(std::vector<Level<T>>& lv, int l, T* x, const T* b, bool x_zero) {
+void Batch::cycle_level(std::vector<Level<T>>& lv, int l, T* x, const T* b, bool x_zero, bool swept) {
     const int L = (int)lv.size();
     if (l == L - 1) {
         coarse_solve<T>(l, b, x);
@@ -781,10 +783,15 @@ void Batch::cycle_level(std::vector<Level<T>>& lv, int l, T* x, const T* b, bool
     };
     T* cur = x;
     T* other = V.xt.get();
-    smooth(cur, other, x_zero);
+    if (!swept) smooth(cur, other, x_zero);
     V.apply_A(cur, gated<Gt>(EpiResidual<T, T>{b, V.r.get()}, gl));
-    rows_op(V.R, V.R16, C.n, V.r.get(), gated<Gt>(EpiStore<T>{C.b.get()}, gc), V.gR);
-    cycle_level<Gt>(lv, l + 1, C.x.get(), C.b.get(), true);
+    const bool next_swept = jt && opts.num_smooth_sweeps == 1 && l + 1 < L - 1;
+    if (next_swept)
+        rows_op(V.R, V.R16, C.n, V.r.get(),
+                gated<Gt>(EpiStoreScale<T>{C.b.get(), C.dinv.get(), C.x.get()}, gc), V.gR);
+    else
+        rows_op(V.R, V.R16, C.n, V.r.get(), gated<Gt>(EpiStore<T>{C.b.get()}, gc), V.gR);
+    cycle_level<Gt>(lv, l + 1, C.x.get(), C.b.get(), true, next_swept);
     T* start = x;
     if (jt && (opts.num_smooth_sweeps & 1)) start = (x == V.xt.get()) ? x : V.xt.get();
     if (cur == start) {

@@ -267,7 +267,7 @@ void bsmooth(const Hierarchy& H, const Level<T>& V, const BLevel<T>& W, T*& cur,
 
 template <typename T>
 void block_cycle_level(Hierarchy& H, std::vector<Level<T>>& lv, std::vector<BLevel<T>>& bl, int l,
-                       T* X, const T* B, bool x_zero, int k) {
+                       T* X, const T* B, bool x_zero, int k, bool swept = false) {
     const int L = (int)lv.size();
     if (l == L - 1) {
         if (H.coarse_n && H.cinv.get())
@@ -295,10 +295,16 @@ void block_cycle_level(Hierarchy& H, std::vector<Level<T>>& lv, std::vector<BLev
     BLevel<T>& WC = bl[l + 1];
     T* cur = X;
     T* other = W.xt.get();
-    bsmooth(H, V, W, cur, other, B, x_zero, k);
+    if (!swept) bsmooth(H, V, W, cur, other, B, x_zero, k);
     apply_A_block(V, W, cur, k, BResidual<T, T>{B, W.r.get()});
-    launch_csr_block(V.R.rowptr, V.R.cols, V.R.vals, C.n, k, W.r.get(), BStore<T>{WC.b.get()}, W.sR);
-    block_cycle_level(H, lv, bl, l + 1, WC.x.get(), WC.b.get(), true, k);
+    const bool next_swept = jacobi_type(H.opts) && H.opts.num_smooth_sweeps == 1 && l + 1 < L - 1 &&
+                            l + 1 != H.dense_from;
+    if (next_swept)
+        launch_csr_block(V.R.rowptr, V.R.cols, V.R.vals, C.n, k, W.r.get(),
+                         BStoreScale<T>{WC.b.get(), C.dinv.get(), WC.x.get()}, W.sR);
+    else
+        launch_csr_block(V.R.rowptr, V.R.cols, V.R.vals, C.n, k, W.r.get(), BStore<T>{WC.b.get()}, W.sR);
+    block_cycle_level(H, lv, bl, l + 1, WC.x.get(), WC.b.get(), true, k, next_swept);
     // x += P x_c into the buffer from which the post-smoothing ping-pong ends in X
     T* start = X;
     if (jacobi_type(H.opts) && (H.opts.num_smooth_sweeps & 1))

@@ -125,6 +125,33 @@ struct BStore {
     bool al16v() const { return al16(y); }
 };
 
+// the restriction with the next level's first sweep (EpiStoreScale, spmv.cuh)
+template <typename T>
+struct BStoreScale {
+    T* y;
+    const T* d;
+    T* x;
+    template <typename A>
+    __device__ void operator()(long i, int c, int k, A s) const {
+        const T v = (T)s;
+        y[i * k + c] = v;
+        x[i * k + c] = v * d[i];
+    }
+    template <int VW, typename A>
+    __device__ void vec(long i, int c0, int k, const A (&s)[VW]) const {
+        T o[VW], w[VW];
+        const T di = __ldg(d + i);
+#pragma unroll
+        for (int v = 0; v < VW; v++) {
+            o[v] = (T)s[v];
+            w[v] = o[v] * di;
+        }
+        vstore<T, VW>(y + i * k + c0, o);
+        vstore<T, VW>(x + i * k + c0, w);
+    }
+    bool al16v() const { return al16(y) && al16(x); }
+};
+
 template <typename TB, typename TY>
 struct BResidual {
     const TB* b;

@@ -843,8 +843,9 @@ void Hierarchy::build_levels(std::vector<Level<T>>& lv) {
             if (!strided_only) V.gA = tune_tiles(V.A, V.A16, V.gA, V.x.get(), V.r.get(), "Atile");
         }
     }
-    // the first sweep from zero fused with the residual, per level, where
-    // one pass over A_l gathering b d beats the sweep and the residual apart
+    // the first sweep from zero fused with the residual at level 0, where
+    // one pass over A_0 gathering b d beats the sweep and the residual apart
+    // (the levels below are swept by their restriction, swept_by_restriction)
     const int rt = opts.relax_type;
     const bool jac1 = ((rt == RB_RELAX_JACOBI && !opts.jacobi_compat) || rt == RB_RELAX_L1JACOBI) &&
                       opts.num_smooth_sweeps == 1;
@@ -857,6 +858,7 @@ void Hierarchy::build_levels(std::vector<Level<T>>& lv) {
             V.fuse_first = force_first == 1;
             continue;
         }
+        if (l > 0) continue;   // swept by the restriction from above
         const std::string key = tune_key(V.dia ? "first_dia" : "first", V.n, V.A.nnz, (int)sizeof(T));
         auto& c = tune_cache();
         auto it = c.m.find(key);
@@ -1266,8 +1268,11 @@ void Hierarchy::smooth(Level<T>& V, T*& cur, T*& other, const T* b, bool x_zero)
 }
 
 
+// swept: x already holds the first sweep's result (the restriction from the
+// level above wrote it).
 template <typename T>
-void Hierarchy::cycle_level(std::vector<Level<T>>& lv, int l, T* x, const T* b, bool x_zero) {
+void Hierarchy::cycle_level(std::vector<Level<T>>& lv, int l, T* x, const T* b, bool x_zero,
+                            bool swept) {
     Level<T>& V = lv[l];
     const int L = (int)lv.size();
     if (l == L - 1) {
@@ -1309,7 +1314,10 @@ void Hierarchy::cycle_level(std::vector<Level<T>>& lv, int l, T* x, const T* b, 
     const int rt = opts.relax_type;
     const bool jacobi_type = (rt == RB_RELAX_JACOBI && !opts.jacobi_compat) || rt == RB_RELAX_L1JACOBI;
     mark(l * kProfSlots + 6);
-    if (x_zero && jacobi_type && opts.num_smooth_sweeps == 1 && V.fuse_first) {
+    if (swept) {
+        mark(l * kProfSlots + 0);
+        V.apply_A(cur, EpiResidual<T, T>{b, V.r.get()});
+    } else if (x_zero && jacobi_type && opts.num_smooth_sweeps == 1 && V.fuse_first) {
         // one sweep from zero, x = D^-1 b, fused with r = b - A x (the
         // profile books the pair as the residual)
         mark(l * kProfSlots + 0);
@@ -1321,10 +1329,14 @@ void Hierarchy::cycle_level(std::vector<Level<T>>& lv, int l, T* x, const T* b, 
         V.apply_A(cur, EpiResidual<T, T>{b, V.r.get()});
     }
     mark(l * kProfSlots + 1);
-    rows_op(V.R, V.R16, C.n, V.r.get(),
-                EpiStore<T>{C.b.get()}, V.gR);
+    const bool next_swept = swept_by_restriction(lv, l + 1);
+    if (next_swept)
+        rows_op(V.R, V.R16, C.n, V.r.get(),
+                EpiStoreScale<T>{C.b.get(), C.dinv.get(), C.x.get()}, V.gR);
+    else
+        rows_op(V.R, V.R16, C.n, V.r.get(), EpiStore<T>{C.b.get()}, V.gR);
     mark(l * kProfSlots + 2);
-    cycle_level(lv, l + 1, C.x.get(), C.b.get(), true);
+    cycle_level(lv, l + 1, C.x.get(), C.b.get(), true, next_swept);
     mark(l * kProfSlots + 6);
     // x += P x_c (par_multilevel.hpp:430), into the buffer from which the
     // post-smoothing ping-pong ends in x
@@ -1345,6 +1357,20 @@ void Hierarchy::cycle_level(std::vector<Level<T>>& lv, int l, T* x, const T* b, 
         RB_CUDA(cudaMemcpyAsync(x, cur, sizeof(T) * V.n, cudaMemcpyDeviceToDevice, stream()));
     }
     mark(l * kProfSlots + 4);
+}
+
+// Every level below the finest that smooths with one Jacobi-type sweep (the
+// coarsest, the dense bottom and the cluster tail do not).  The sweep from
+// zero is one multiply a row where the restriction's rows are written: as a
+// launch of its own it took 3 to 8 us a level, and fused with the residual
+// (EpiFirstResidual, still the choice at level 0 and where
+// RAPTOR_B200_FUSE_FIRST=1 asks for it) a second gather an entry.
+template <typename T>
+bool Hierarchy::swept_by_restriction(const std::vector<Level<T>>& lv, int l) const {
+    const int rt = opts.relax_type;
+    const bool jacobi_type = (rt == RB_RELAX_JACOBI && !opts.jacobi_compat) || rt == RB_RELAX_L1JACOBI;
+    return jacobi_type && opts.num_smooth_sweeps == 1 && l < (int)lv.size() - 1 && l != dense_from &&
+           l != tail_from && !lv[l].fuse_first;
 }
 
 void Hierarchy::mark(int slot) {

@@ -223,7 +223,11 @@ struct Hierarchy {
     template <typename T>
     void smooth(Level<T>& V, T*& cur, T*& other, const T* b, bool x_zero);
     template <typename T>
-    void cycle_level(std::vector<Level<T>>& lv, int l, T* x, const T* b, bool x_zero);
+    void cycle_level(std::vector<Level<T>>& lv, int l, T* x, const T* b, bool x_zero,
+                     bool swept = false);
+    // whether the restriction to level l also does its first sweep
+    template <typename T>
+    bool swept_by_restriction(const std::vector<Level<T>>& lv, int l) const;
     void cycle64(double* x, const double* b, bool x_zero);
     void cycle(double* x, const double* b, bool x_zero);
     void run_graph(const std::string& key, const std::function<void()>& fn);

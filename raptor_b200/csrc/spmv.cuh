@@ -107,6 +107,30 @@ struct EpiStore {
     __device__ void operator()(long i, A s, double&) const { y[i] = (TY)s; }
 };
 
+// The restriction with the next level's first sweep from a zero iterate: y =
+// b_c, x = D^-1 b_c (k_scale_first's product), so that the level starts at
+// its residual.
+template <typename T>
+struct EpiStoreScale {
+    T* y;
+    const T* d;
+    T* x;
+    template <typename A>
+    __device__ void operator()(long i, A s, double&) const {
+        const T v = (T)s;
+        y[i] = v;
+        x[i] = (T)(v * d[i]);
+    }
+    struct Pre { T d; };
+    __device__ Pre pre(long i) const { return Pre{__ldg(d + i)}; }
+    template <typename A>
+    __device__ void post(long i, A s, double&, const Pre& p) const {
+        const T v = (T)s;
+        y[i] = v;
+        x[i] = (T)(v * p.d);
+    }
+};
+
 template <typename TB, typename TY>
 struct EpiResidual {
     const TB* b;
