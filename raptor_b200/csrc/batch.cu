@@ -626,7 +626,7 @@ void Batch::setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o) {
             const int nc = M[depth[s] - 1].A->n_rows, nd = M[cut[s] - 1].A->n_rows;
             if (!nc || !nd) continue;
             DevArray<double> inv((size_t)nc * nc), B;
-            k_lu_invert<<<1, 256, sizeof(double) * nc, stream()>>>(nc, lu.get() + luo[s],
+            k_lu_invert<<<nc, 64, sizeof(double) * nc, stream()>>>(nc, lu.get() + luo[s],
                                                                   piv.get() + pivo[s], inv.get());
             RB_CHECK_LAUNCH();
             if (o.precision == RB_PREC_FP32) form_dense_bottom<float>(M, o, cut[s] - 1, inv.get(), nullptr, B);

@@ -338,11 +338,12 @@ __global__ void k_lu_solve(int n, const double* __restrict__ lu, const int* __re
 // no sequential substitution steps.
 constexpr int kCoarseInvMax = 512;
 
-// inv (column-major, n x n) = the inverse of the matrix factored in lu/piv.
+// inv (column-major, n x n) = the inverse of the matrix factored in lu/piv, a
+// block a column (one block for all of them took 0.35 ms for 41 columns).
 static __global__ void k_lu_invert(int n, const double* __restrict__ lu, const int* __restrict__ piv,
                                    double* __restrict__ inv) {
     extern __shared__ double y[];
-    for (int c = 0; c < n; c++) {
+    for (int c = blockIdx.x; c < n; c += gridDim.x) {
         for (int i = threadIdx.x; i < n; i += blockDim.x) y[i] = (i == c) ? 1.0 : 0.0;
         __syncthreads();
         if (threadIdx.x == 0)

@@ -96,16 +96,22 @@ static __global__ void k_dense_from_inverse(int n, const double* __restrict__ in
     if (c < n) out[(size_t)i * n + c] = inv[(size_t)c * n + i];
 }
 
-// M = I - A D, one thread a row (M zeroed before)
+// M = I - A D, one warp a row (M zeroed before; a thread a row waited for its
+// entries one by one).  The adds are atomic for a row that names a column
+// twice; where none does, as in every product matrix, each entry has one.
 template <typename T>
 __global__ void k_dense_first_residual(int n, const int* __restrict__ rp, const int* __restrict__ ci,
                                        const double* __restrict__ cv, const T* __restrict__ d,
                                        double* M) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= n) return;
     double* row = M + (size_t)i * n;
-    row[i] = 1.0;
-    for (int j = rp[i]; j < rp[i + 1]; j++) row[ci[j]] -= cv[j] * (double)d[ci[j]];
+    if (lane == 0) row[i] = 1.0;
+    __syncwarp();
+    for (int j = rp[i] + lane; j < rp[i + 1]; j += 32) {
+        const int c = ci[j];
+        atomicAdd(row + c, -(cv[j] * (double)d[c]));
+    }
 }
 
 // M = the CSR matrix, dense with m columns (M zeroed before)

@@ -904,7 +904,7 @@ void Hierarchy::build_cycle_data() {
     cinv.release();
     if (coarse_n > 0 && coarse_n <= kCoarseInvMax) {
         cinv.alloc((size_t)coarse_n * coarse_n);
-        k_lu_invert<<<1, 256, sizeof(double) * coarse_n, stream()>>>(coarse_n, lu.get(), piv.get(),
+        k_lu_invert<<<coarse_n, 64, sizeof(double) * coarse_n, stream()>>>(coarse_n, lu.get(), piv.get(),
                                                                        cinv.get());
         RB_CHECK_LAUNCH();
     }
@@ -1031,7 +1031,7 @@ void form_dense_bottom(const std::vector<MasterLevel>& master, const rb_amg_opts
             k_dense_copy<<<grid_for(nc, 128), 128, 0, stream()>>>(nc, n, rrp, rci, rcv, Tm.get());
         } else {
             W.zero();
-            k_dense_first_residual<T><<<grid_for(n, 128), 128, 0, stream()>>>(n, arp, aci, acv, d, W.get());
+            k_dense_first_residual<T><<<grid_for((long)n * 32, 128), 128, 0, stream()>>>(n, arp, aci, acv, d, W.get());
             RB_CHECK_LAUNCH();
             k_dense_spmm<0, T><<<dim3(cols(n), nc), 256, 0, stream()>>>(n, rrp, rci, rcv, W.get(), d, Tm.get());
         }
