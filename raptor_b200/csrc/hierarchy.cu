@@ -171,6 +171,12 @@ std::string tune_key(const char* op, long n, long long nnz, int vbytes) {
     return b;
 }
 
+// Operators of fewer rows are not timed: every schedule takes the 2 to 3 us of
+// a launch there, so the timing picked one at random -- and with it the order
+// of its sums, which a long CG history at 1e-10 shows (100^2) -- for a
+// first setup longer by its launches.
+constexpr int kTuneRows = 16384;
+
 // Time the row kernel for each group width and keep the fastest.
 template <typename T>
 static int autotune_group_timed(const CsrView<T>& M, T* xin, T* yout, bool strided);
@@ -179,7 +185,7 @@ static int autotune_group_timed(const CsrView<T>& M, T* xin, T* yout, bool strid
 template <typename T>
 static int autotune_group(const CsrView<T>& M, T* xin, T* yout, const char* op = "rows",
                           bool strided = false) {
-    if (M.n_rows < 4096) return pick_group(M.n_rows, M.nnz);
+    if (M.n_rows < kTuneRows) return pick_group(M.n_rows, M.nnz);
     const std::string key = tune_key((strided ? std::string("s") + op : std::string(op)).c_str(),
                                      M.n_rows, M.nnz, (int)sizeof(T));
     auto& c = tune_cache();
@@ -219,7 +225,7 @@ static void tune_idx16(const CsrView<T>& M, Idx16& I, int G, const T* xin, T* yo
     // the rows allow it (any size), unset lets the timing decide
     const char* env = getenv("RAPTOR_B200_IDX16");
     const int force = (env && env[0] == '0') ? 0 : (env && env[0] == '1') ? 1 : -1;
-    if (force == 0 || M.nnz == 0 || (force < 0 && M.n_rows < 4096)) return;
+    if (force == 0 || M.nnz == 0 || (force < 0 && M.n_rows < kTuneRows)) return;
     const std::string key = tune_key(op, M.n_rows, M.nnz, (int)sizeof(T));
     auto& c = tune_cache();
     auto it = c.m.find(key);
@@ -279,7 +285,7 @@ static int tune_tiles(const CsrView<T>& M, Idx16& I, int G, const T* xin, T* you
     I.tchunks = 0;
     const char* env = getenv("RAPTOR_B200_TILED");
     const int force = (env && env[0] == '0') ? 0 : (env && env[0] == '1') ? 1 : -1;
-    if (force == 0 || M.nnz == 0 || (force < 0 && M.n_rows < 4096)) return G;
+    if (force == 0 || M.nnz == 0 || (force < 0 && M.n_rows < kTuneRows)) return G;
     const std::string key = tune_key(op, M.n_rows, M.nnz, (int)sizeof(T));
     auto& c = tune_cache();
     auto it = c.m.find(key);
@@ -806,7 +812,9 @@ void Hierarchy::build_levels(std::vector<Level<T>>& lv) {
             const std::string key = tune_key("A_dia", V.n, V.A.nnz, (int)sizeof(T));
             auto& c = tune_cache();
             auto it = c.m.find(key);
-            if (it != c.m.end()) {
+            if (V.n < kTuneRows) {
+                V.dia = true;
+            } else if (it != c.m.end()) {
                 V.dia = it->second != 0;
             } else {
                 const size_t xb = sizeof(T) * (size_t)V.n;
