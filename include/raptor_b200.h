@@ -269,10 +269,12 @@ typedef struct rb_amg_opts {
     int precision;            /* RB_PREC_FP64 / RB_PREC_FP32 */
     int jacobi_compat;        /* 1: Jacobi leaves x unchanged, as par_relax.cpp:127,146 does */
     int seed_offset;          /* first_local_row in srand(2448422 + first_local_row) */
-    int fuse_coarse;          /* 1 (default): the bottom levels of the cycle run as one launch of one
-                                 thread-block cluster, from the start level that times fastest
-                                 (none if no start beats separate launches); 0: never;
-                                 k >= 2: from level k-1 if that level qualifies */
+    int fuse_coarse;          /* 1 (default): the bottom levels of the cycle run as one dense product
+                                 formed at setup, from the first level whose matrix fits (Jacobi-type
+                                 smoothing with one sweep); where it does not apply, as one launch of
+                                 one thread-block cluster, from the start level that times fastest
+                                 (none if no start beats separate launches); 0: neither;
+                                 k >= 2: the cluster from level k-1 if that level qualifies */
     int use_graphs;           /* 1: replay cycles / Krylov iterations from CUDA graphs */
     int const_coef;           /* 1 (default): a diagonal-storage level whose diagonals each hold one
                                  value is read as a mask a row plus those values (same results);
