@@ -93,7 +93,15 @@ void* device_alloc(size_t bytes, bool* pooled) {
     cudaStream_t s = stream();
     if (bytes >= kPoolLargest || capturing(s)) {
         *pooled = false;
-        RB_CUDA(cudaMalloc(&p, bytes));
+        cudaError_t e = cudaMalloc(&p, bytes);
+        if (e == cudaErrorMemoryAllocation && !capturing(s)) {   // what the pool keeps may be what is missing
+            (void)cudaGetLastError();
+            RB_CUDA(cudaDeviceSynchronize());
+            RB_CUDA(cudaMemPoolTrimTo(pool_of_device(), 0));
+            e = cudaMalloc(&p, bytes);
+        }
+        if (e != cudaSuccess) (void)cudaGetLastError();
+        RB_CUDA(e);
         return p;
     }
     *pooled = true;
