@@ -271,37 +271,92 @@ long long exclusive_scan(const int* in, int* out, int n) {
 // finds its place by counting the entries before it, so the row is read and
 // written once, coalesced (an insertion sort in global memory, a thread a
 // row: 2.97 ms of a 64^3 27-point setup, 0.93 ms its largest call; this way
-// 0.29 and 0.13).  Rows
-// longer than the group's share of kSortCap entries keep the insertion sort.
-constexpr int kSortCap = 384;   // entries a warp stages (12 bytes each)
+// 0.29 and 0.13).  Rows longer than the group's share of kSortCap entries are
+// then sorted by the whole block, below: an insertion sort by one lane took
+// 1.5 s for the column of 9000 entries that a transpose leaves in any order.
+constexpr int kSortCap = 384;                    // entries a warp stages (12 bytes each)
+constexpr int kSortHalf = 8 * kSortCap / 2;      // a run of a long row: half of what a block stages
 
-__device__ void insertion_sort_row(int i, int s, int e, int* cols, double* vals, int diag_first) {
-    for (int j = s + 1; j < e; j++) {
-        int c = cols[j];
-        double v = vals[j];
-        int k = j - 1;
-        while (k >= s && cols[k] > c) {
-            cols[k + 1] = cols[k];
-            vals[k + 1] = vals[k];
-            k--;
+// One long row by the block: runs of kSortHalf entries sorted by rank, then
+// odd-even rounds that merge neighbouring runs in place (as many rounds as
+// runs; pairs in order already are left).  Both are stable, and no scratch
+// beyond the block's shared memory is needed.
+__device__ void block_sort_row(int i, int s, int m, int* cols, double* vals, int diag_first,
+                               double* sv, int* sc) {
+    const int tid = threadIdx.x, nth = blockDim.x;
+    for (int lo = 0; lo < m; lo += kSortHalf) {
+        const int len = min(kSortHalf, m - lo);
+        for (int t = tid; t < len; t += nth) {
+            sc[t] = cols[s + lo + t];
+            sv[t] = vals[s + lo + t];
         }
-        cols[k + 1] = c;
-        vals[k + 1] = v;
+        __syncthreads();
+        for (int t = tid; t < len; t += nth) {
+            const int c = sc[t];
+            int rank = 0;
+            for (int j = 0; j < len; j++) rank += sc[j] < c || (sc[j] == c && j < t);
+            cols[s + lo + rank] = c;
+            vals[s + lo + rank] = sv[t];
+        }
+        __syncthreads();
     }
-    if (diag_first) {
-        for (int j = s; j < e; j++) {
-            if (cols[j] == i) {
-                double t = vals[j];
-                for (int k = j; k > s; k--) {
-                    cols[k] = cols[k - 1];
-                    vals[k] = vals[k - 1];
-                }
-                cols[s] = i;
-                vals[s] = t;
-                break;
+    const int runs = (m + kSortHalf - 1) / kSortHalf;
+    for (int round = 0; round < runs; round++)
+        for (int r = round & 1; r + 1 < runs; r += 2) {
+            const int lo = r * kSortHalf, nr = min(kSortHalf, m - lo - kSortHalf);
+            for (int t = tid; t < kSortHalf + nr; t += nth) {
+                sc[t] = cols[s + lo + t];
+                sv[t] = vals[s + lo + t];
             }
+            __syncthreads();
+            if (sc[kSortHalf - 1] > sc[kSortHalf])
+                for (int t = tid; t < kSortHalf + nr; t += nth) {
+                    const int c = sc[t];
+                    const bool left = t < kSortHalf;
+                    // entries of the other run that come before: smaller
+                    // ones, and from the right also equal ones
+                    const int* o = left ? sc + kSortHalf : sc;
+                    int a = 0, b = left ? nr : kSortHalf;
+                    while (a < b) {
+                        const int h = (a + b) >> 1;
+                        if (o[h] < c || (!left && o[h] == c)) a = h + 1;
+                        else b = h;
+                    }
+                    const int rank = (left ? t : t - kSortHalf) + a;
+                    cols[s + lo + rank] = c;
+                    vals[s + lo + rank] = sv[t];
+                }
+            __syncthreads();
         }
+    if (!diag_first) return;
+    int a = 0, b = m;   // the first entry of the diagonal
+    while (a < b) {
+        const int h = (a + b) >> 1;
+        if (cols[s + h] < i) a = h + 1;
+        else b = h;
     }
+    const bool has = a < m && cols[s + a] == i;
+    const double dv = has ? vals[s + a] : 0.0;
+    __syncthreads();
+    if (!has) return;
+    for (int hi = a; hi > 0; hi -= 2 * kSortHalf) {   // entries before it, one place up
+        const int lo = max(0, hi - 2 * kSortHalf);
+        for (int t = tid; t < hi - lo; t += nth) {
+            sc[t] = cols[s + lo + t];
+            sv[t] = vals[s + lo + t];
+        }
+        __syncthreads();
+        for (int t = tid; t < hi - lo; t += nth) {
+            cols[s + lo + t + 1] = sc[t];
+            vals[s + lo + t + 1] = sv[t];
+        }
+        __syncthreads();
+    }
+    if (tid == 0) {
+        cols[s] = i;
+        vals[s] = dv;
+    }
+    __syncthreads();
 }
 
 template <int G>
@@ -314,36 +369,42 @@ k_sort_rows(int n, const int* __restrict__ rp, int* cols, double* vals, int diag
     const int gl = lane & (G - 1), sub = lane / G;
     const unsigned mask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (lane & ~(G - 1));
     const long i = (((long)blockIdx.x * blockDim.x + threadIdx.x) / G);
-    if (i >= n) return;
-    const int s = rp[i], m = rp[i + 1] - s;
-    if (m <= 1) return;
-    if (m > CAP) {
-        if (gl == 0) insertion_sort_row((int)i, s, s + m, cols, vals, diag_first);
-        return;
+    int s = 0, m = 0;
+    if (i < n) {
+        s = rp[i];
+        m = rp[i + 1] - s;
     }
-    double* sv = sval[wid] + sub * CAP;
-    int* sc = scol[wid] + sub * CAP;
-    for (int t = gl; t < m; t += G) {
-        sc[t] = cols[s + t];
-        sv[t] = vals[s + t];
+    if (m > 1 && m <= CAP) {
+        double* sv = sval[wid] + sub * CAP;
+        int* sc = scol[wid] + sub * CAP;
+        for (int t = gl; t < m; t += G) {
+            sc[t] = cols[s + t];
+            sv[t] = vals[s + t];
+        }
+        __syncwarp(mask);
+        for (int t = gl; t < m; t += G) {
+            const int c = sc[t];
+            int rank = 0, equal_before = 0, diag = 0;
+            for (int j = 0; j < m; j++) {
+                const int cj = sc[j];
+                const int eq = cj == c && j < t;
+                rank += cj < c || eq;
+                equal_before |= eq;
+                diag |= cj == (int)i;
+            }
+            if (diag_first && diag) {
+                if (c == (int)i && !equal_before) rank = 0;
+                else if (c < (int)i) rank++;
+            }
+            cols[s + rank] = c;
+            vals[s + rank] = sv[t];
+        }
     }
-    __syncwarp(mask);
-    for (int t = gl; t < m; t += G) {
-        const int c = sc[t];
-        int rank = 0, equal_before = 0, diag = 0;
-        for (int j = 0; j < m; j++) {
-            const int cj = sc[j];
-            const int eq = cj == c && j < t;
-            rank += cj < c || eq;
-            equal_before |= eq;
-            diag |= cj == (int)i;
-        }
-        if (diag_first && diag) {
-            if (c == (int)i && !equal_before) rank = 0;
-            else if (c < (int)i) rank++;
-        }
-        cols[s + rank] = c;
-        vals[s + rank] = sv[t];
+    if (!__syncthreads_or(m > CAP)) return;
+    const long first = (long)blockIdx.x * blockDim.x / G;
+    for (long k = first; k < first + blockDim.x / G && k < n; k++) {
+        const int ks = rp[k], km = rp[k + 1] - ks;
+        if (km > CAP) block_sort_row((int)k, ks, km, cols, vals, diag_first, sval[0], scol[0]);
     }
 }
 

@@ -2,7 +2,8 @@
 products whose rows overflow the first key table (192 and 768 distinct
 columns), fill each table of the numeric pass (64, 128, 256, 2048 and more)
 and have long rows of A or of B; row sorts at the staging area's capacity (96
-and 384 entries), with and without a diagonal, and with repeated columns;
+and 384 entries a group, runs of 1536 for longer rows), with and without a
+diagonal, and with repeated columns;
 extended interpolation with sets of more than 64 and more than 256 points.
 Products and interpolation are compared bit for bit with sums in the same
 order."""
@@ -60,7 +61,8 @@ def test_row_sort(mean):
     rng = np.random.default_rng(mean)
     n = 700
     lens = rng.integers(0, 2 * mean + 1, n)
-    lens[rng.choice(n, 8, replace=False)] = [0, 1, 95, 96, 97, 383, 384, 385]
+    lens[rng.choice(n, 14, replace=False)] = [0, 1, 95, 96, 97, 383, 384, 385,
+                                              1535, 1536, 1537, 3072, 3073, 9001]
     rowptr = np.zeros(n + 1, np.int32)
     rowptr[1:] = np.cumsum(lens)
     cols = rng.integers(0, n, rowptr[-1]).astype(np.int32)      # repeated columns too
