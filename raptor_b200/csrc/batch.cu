@@ -482,7 +482,7 @@ void Batch::choose_cut(const std::vector<std::unique_ptr<Hierarchy>>& sys, std::
         for (int s = 0; s < n; s++) {
             const int m = sys[s]->master[c[s] - 1].A->n_rows;
             if (at) (*at)[s] = t;
-            t += (long long)m * dense_ld<double>(m);
+            t += (long long)m * dense_ld(m);
         }
         if (at) (*at)[n] = t;
         return t * (long long)sizeof(double);
@@ -631,9 +631,8 @@ void Batch::setup(int n, const rb_csr_s* const* mats, const rb_amg_opts& o) {
             RB_CHECK_LAUNCH();
             if (o.precision == RB_PREC_FP32) form_dense_bottom<float>(M, o, cut[s] - 1, inv.get(), nullptr, B);
             else form_dense_bottom<double>(M, o, cut[s] - 1, inv.get(), nullptr, B);
-            const int ld = dense_ld<double>(nd);
-            k_dense_store<double><<<dim3((ld + 255) / 256, nd), 256, 0, stream()>>>(nd, ld, B.get(),
-                                                                                    dense.get() + doff[s]);
+            const int ld = dense_ld(nd);
+            k_dense_store<<<dim3((ld + 255) / 256, nd), 256, 0, stream()>>>(nd, ld, B.get(), dense.get() + doff[s]);
             RB_CHECK_LAUNCH();
         }
     }

@@ -280,12 +280,9 @@ void block_cycle_level(Hierarchy& H, std::vector<Level<T>>& lv, std::vector<BLev
         return;
     }
     if (l == H.dense_from) {
-        const T* M;
-        if constexpr (std::is_same<T, float>::value) M = H.dense32.get();
-        else M = H.dense64.get();
         const int n = lv[l].n;
         k_dense_mm<T><<<dim3((n + 3) / 4, (k + kDenseCols - 1) / kDenseCols), 128, 0, stream()>>>(
-            n, H.dense_ld_, M, k, B, X);
+            n, H.dense_ld_, H.dense.get(), k, B, X);
         RB_CHECK_LAUNCH();
         return;
     }

@@ -4,18 +4,24 @@
 // right-hand side: x_f = B b_f with a fixed n_f x n_f matrix B.  Level by
 // level it costs five small kernels a level (2 us of launch and drain each,
 // 4 to 17 us for the coarsest solve or the cluster tail), whatever their
-// size; B of a level of a thousand rows is 4 MB in FP32, which the L2 holds,
-// and one product with it takes about 3 us.  Setup forms B once, in FP64 from
-// the FP64 hierarchy, upwards from the inverse of the coarsest matrix:
+// size; one product with B takes 3.9 us (100^2; 192^3: 4.5) to 8.7
+// us (1024^2), for 8 columns 27 us (96^3, smoothed aggregation).  Setup forms B
+// once, in FP64 from the FP64 hierarchy, upwards from the inverse of the
+// coarsest matrix:
 //
 //     T = R (I - A D)         restriction of the first sweep's residual
 //     E = B_c T               the level below
 //     X = D + P E             first sweep plus coarse correction
 //     B = X + D (I - A X)     post-sweep
 //
-// with D the smoother's scaled inverse diagonal (no sweeps: B = P B_c R),
-// and rounds it once to the cycle's precision.  The product accumulates in
-// FP64.
+// with D the smoother's scaled inverse diagonal (no sweeps: B = P B_c R).
+// B stays in FP64 under an FP32 cycle too, as the coarsest inverse does: on a
+// nearly singular operator its entries are dominated by the large multiple of
+// the near-null vector's projector, and rounded to FP32 they lose what the
+// cycle does to everything else (graph Laplacian + 1e-7 on 40^3: error off
+// the constant 2e-4, in FP64 8e-8).  With the 16 MB below it costs an FP32
+// cycle nothing (192^3 PCG 8.42 and 8.50 ms, 1024^2 12.6 and 12.2, runs of one
+// side 2.5% apart; 32 MB and its 2048 rows: 8.51 and 12.5).
 #pragma once
 
 #include "rb_common.cuh"
@@ -27,26 +33,20 @@ namespace rb {
 // two of the launches it replaces take.
 constexpr size_t kDenseBytes = (size_t)16 << 20;
 
-// Row length of B in elements of T: rows start on 16-byte boundaries.
-template <typename T>
-inline int dense_ld(int n) {
-    constexpr int v = 16 / sizeof(T);
-    return (n + v - 1) / v * v;
-}
+// Row length of B: rows start on 16-byte boundaries.
+inline int dense_ld(int n) { return (n + 1) & ~1; }
 
 // Row `row` of B b for one warp: 16 bytes a lane and step, rows padded with
 // zeros to ld, b read only below n; every lane gets the sum.
-template <typename TM, typename T>
-__device__ __forceinline__ double dense_row(int n, int ld, const TM* __restrict__ r,
+template <typename T>
+__device__ __forceinline__ double dense_row(int n, int ld, const double* __restrict__ r,
                                             const T* __restrict__ b) {
-    constexpr int V = 16 / sizeof(TM);
     double s = 0.0;
 #pragma unroll 4
-    for (int j = (threadIdx.x & 31) * V; j < ld; j += 32 * V) {
-        TM a[V];
-        *reinterpret_cast<uint4*>(a) = __ldg(reinterpret_cast<const uint4*>(r + j));
-#pragma unroll
-        for (int v = 0; v < V; v++) s += (double)a[v] * (j + v < n ? (double)__ldg(b + j + v) : 0.0);
+    for (int j = (threadIdx.x & 31) * 2; j < ld; j += 64) {
+        const double2 a = __ldg(reinterpret_cast<const double2*>(r + j));
+        s += a.x * (double)__ldg(b + j);
+        s += a.y * (j + 1 < n ? (double)__ldg(b + j + 1) : 0.0);
     }
     return warp_sum(s);
 }
@@ -54,7 +54,7 @@ __device__ __forceinline__ double dense_row(int n, int ld, const TM* __restrict_
 // x = B b, one warp a row
 template <typename T>
 __global__ void __launch_bounds__(128)
-k_dense_mv(int n, int ld, const T* __restrict__ B, const T* __restrict__ b, T* __restrict__ x) {
+k_dense_mv(int n, int ld, const double* __restrict__ B, const T* __restrict__ b, T* __restrict__ x) {
     const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (row >= n) return;
     const double s = dense_row(n, ld, B + (size_t)row * ld, b);
@@ -66,16 +66,16 @@ k_dense_mv(int n, int ld, const T* __restrict__ B, const T* __restrict__ b, T* _
 constexpr int kDenseCols = 8;
 template <typename T>
 __global__ void __launch_bounds__(128)
-k_dense_mm(int n, int ld, const T* __restrict__ B, int k, const T* __restrict__ b,
+k_dense_mm(int n, int ld, const double* __restrict__ B, int k, const T* __restrict__ b,
            T* __restrict__ x) {
     const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     const int c0 = blockIdx.y * kDenseCols;
     if (row >= n) return;
-    const T* r = B + (size_t)row * ld;
+    const double* r = B + (size_t)row * ld;
     double s[kDenseCols] = {};
 #pragma unroll 2
     for (int j = lane; j < n; j += 32) {
-        const double a = (double)__ldg(r + j);
+        const double a = __ldg(r + j);
         T v[kDenseCols];
 #pragma unroll
         for (int c = 0; c < kDenseCols; c++) v[c] = c0 + c < k ? __ldg(b + (size_t)j * k + c0 + c) : T(0);
@@ -180,11 +180,11 @@ k_dense_gemm(int n, int m, const double* __restrict__ A, const double* __restric
         }
 }
 
-// B in the cycle precision, rows padded to ld
-template <typename T>
-__global__ void k_dense_store(int n, int ld, const double* __restrict__ in, T* __restrict__ out) {
+// B with its rows padded to ld
+static __global__ void k_dense_store(int n, int ld, const double* __restrict__ in,
+                                     double* __restrict__ out) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
-    if (c < ld) out[(size_t)i * ld + c] = c < n ? (T)in[(size_t)i * n + c] : T(0);
+    if (c < ld) out[(size_t)i * ld + c] = c < n ? in[(size_t)i * n + c] : 0.0;
 }
 
 }  // namespace rb

@@ -958,8 +958,8 @@ void Hierarchy::build_cycle_data() {
 
 void Hierarchy::build_bottom() {
     release_graphs();
-    if (opts.precision == RB_PREC_FP32) build_dense(lv32, dense32);
-    else build_dense(lv64, dense64);
+    if (opts.precision == RB_PREC_FP32) build_dense(lv32);
+    else build_dense(lv64);
     if (dense_from >= 0) {
         tail_from = -1;
         tail_ms.clear();
@@ -977,15 +977,15 @@ void Hierarchy::build_bottom() {
 // leaves it off).  Always taken where it applies: it replaces at least six
 // launches by one.
 template <typename T>
-void Hierarchy::build_dense(std::vector<Level<T>>& lv, DevArray<T>& B) {
+void Hierarchy::build_dense(std::vector<Level<T>>& lv) {
     dense_from = -1;
-    B.release();
+    dense.release();
     const int L = (int)lv.size();
     if (opts.fuse_coarse != 1 || !dense_bottom_applies(opts) || L < 3 || !cinv.get()) return;
     int f = -1;
     for (int l = L - 2; l >= 1; l--) {
         const size_t n = (size_t)lv[l].n;
-        if (n == 0 || n * (size_t)dense_ld<T>(lv[l].n) * sizeof(T) > kDenseBytes) break;
+        if (n == 0 || n * (size_t)dense_ld(lv[l].n) * sizeof(double) > kDenseBytes) break;
         f = l;
     }
     if (f < 0) return;
@@ -994,9 +994,9 @@ void Hierarchy::build_dense(std::vector<Level<T>>& lv, DevArray<T>& B) {
     DevArray<double> Bf;
     form_dense_bottom<T>(master, opts, f, cinv.get(), dinv.data(), Bf);
     const int n = lv[f].n;
-    dense_ld_ = dense_ld<T>(n);
-    B.alloc((size_t)n * dense_ld_);
-    k_dense_store<T><<<dim3((dense_ld_ + 255) / 256, n), 256, 0, stream()>>>(n, dense_ld_, Bf.get(), B.get());
+    dense_ld_ = dense_ld(n);
+    dense.alloc((size_t)n * dense_ld_);
+    k_dense_store<<<dim3((dense_ld_ + 255) / 256, n), 256, 0, stream()>>>(n, dense_ld_, Bf.get(), dense.get());
     RB_CHECK_LAUNCH();
     dense_from = f;
 }
@@ -1298,11 +1298,8 @@ void Hierarchy::cycle_level(std::vector<Level<T>>& lv, int l, T* x, const T* b, 
     if (l == dense_from) {
         // (from a zero guess, as every level below the finest starts; the
         // profile books it as level dense_from's slot 5)
-        const T* B;
-        if constexpr (std::is_same<T, float>::value) B = dense32.get();
-        else B = dense64.get();
         mark(l * kProfSlots + 6);
-        k_dense_mv<T><<<(V.n + 3) / 4, 128, 0, stream()>>>(V.n, dense_ld_, B, b, x);
+        k_dense_mv<T><<<(V.n + 3) / 4, 128, 0, stream()>>>(V.n, dense_ld_, dense.get(), b, x);
         RB_CHECK_LAUNCH();
         mark(l * kProfSlots + 5);
         return;

@@ -185,10 +185,9 @@ struct Hierarchy {
     // (dense_bottom.cuh); dense_from = -1: off
     int dense_from = -1;
     int dense_ld_ = 0;
-    DevArray<double> dense64;
-    DevArray<float> dense32;
+    DevArray<double> dense;
     template <typename T>
-    void build_dense(std::vector<Level<T>>& lv, DevArray<T>& B);
+    void build_dense(std::vector<Level<T>>& lv);
     void build_bottom();   // the dense product where it applies, else the timed tail
     std::map<std::string, cudaGraphExec_t> graphs;
     std::map<std::string, long long> graph_kernels;
