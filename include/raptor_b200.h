@@ -129,7 +129,9 @@ int rb_spmv(rb_csr A, rb_vec x, rb_vec b);
 int rb_residual(rb_csr A, rb_vec x, rb_vec b, rb_vec r);
 /* ParMatrix::mult_T, b = A^T x (par_spmv.cpp:157-187 -> spmv.cpp:150-163).
  * The first call on a matrix builds and keeps A^T's pattern on the handle;
- * later calls gather A's current values through it. */
+ * later calls gather A's current values through it.  Unlike the other
+ * products, which are only ordered on the library's stream, it returns when
+ * the result is complete. */
 int rb_spmv_T(rb_csr A, rb_vec x, rb_vec b);
 /* ParMatrix::mult_append, b += A x (par_spmv.cpp:91-125 -> spmv.cpp:88-103) */
 int rb_spmv_append(rb_csr A, rb_vec x, rb_vec b);

@@ -373,10 +373,12 @@ int rb_spmv_T(rb_csr A, rb_vec x, rb_vec b) {
         NEED(A); NEED(x); NEED(b);
         RB_REQUIRE(x->n == A->n_rows && b->n == A->n_cols, "spmv_T: sizes do not match");
         // a gather over A^T's pattern, cached on the handle: deterministic,
-        // no atomics, no allocation after the first call; ordered on the
-        // library's stream like the other products (the host used to wait
-        // here: 8 of the 27 us of four products on 10,000 rows)
+        // no atomics, no allocation after the first call.  The result is
+        // complete on return, on any stream of the caller's: the wait is 8 of
+        // the 27 us of four products on 10,000 rows, and without it a caller
+        // that reads b on a stream of its own races with the product
         spmv_T64(*A, x->v.get(), b->v.get());
+        RB_CUDA(cudaStreamSynchronize(stream()));
         return RB_OK;
     });
 }

@@ -57,6 +57,39 @@ def test_products_with_long_rows_and_columns(n, m, mean, special):
     assert np.all(np.abs(t.numpy() - wantT) <= eps * (np.bincount(cols, minlength=m) + 2) * scaleT + 1e-300)
 
 
+def test_transposed_product_is_complete_on_return():
+    """Whatever was queued before it on the stream: the caller may read the
+    result on another stream at once (the first call also builds the map)."""
+    torch = pytest.importorskip("torch")
+    A = rb.par_stencil_grid(rb.diffusion_stencil_2d(0.1, 0.4), [70, 90])
+    n = A.global_num_rows
+    uh = np.random.default_rng(5).uniform(-1, 1, n)
+    u, t = rb.ParVector(n, values=uh), rb.ParVector(n)
+    s, mine = torch.cuda.Stream(), torch.cuda.Stream()
+    busy = torch.zeros(1 << 26, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    got = []
+    try:
+        rb.set_stream(s.cuda_stream)
+        for rep in range(3):
+            with torch.cuda.stream(s):
+                for _ in range(20):
+                    busy += 1.0      # about 3 ms of work ahead of the product
+            A.mult_T(u, t)
+            assert s.query()
+            with torch.cuda.stream(mine):
+                got.append(t.torch_view().clone())
+            mine.synchronize()
+            t.set_const_value(0.0)
+    finally:
+        rb.synchronize()
+        rb.set_stream(0)
+    b = rb.ParVector(n)
+    A.mult(u, b)                     # the stencil is symmetric
+    for g in got:
+        np.testing.assert_allclose(g.cpu().numpy(), b.numpy(), rtol=1e-13, atol=1e-13)
+
+
 @pytest.mark.parametrize("prec", [rb.FP64, rb.FP32], ids=["fp64", "fp32"])
 @pytest.mark.parametrize("k", [4, 8, 12, 16, 24])
 def test_block_cycle_with_split_rows(prec, k):
