@@ -61,7 +61,7 @@ def test_transposed_product_is_complete_on_return():
     """Whatever was queued before it on the stream: the caller may read the
     result on another stream at once (the first call also builds the map)."""
     torch = pytest.importorskip("torch")
-    A = rb.par_stencil_grid(rb.diffusion_stencil_2d(0.1, 0.4), [70, 90])
+    A = rb.par_stencil_grid(rb.diffusion_stencil_2d(0.1, 0.4), [80, 80])
     n = A.global_num_rows
     uh = np.random.default_rng(5).uniform(-1, 1, n)
     u, t = rb.ParVector(n, values=uh), rb.ParVector(n)
@@ -85,7 +85,7 @@ def test_transposed_product_is_complete_on_return():
         rb.synchronize()
         rb.set_stream(0)
     b = rb.ParVector(n)
-    A.mult(u, b)                     # the stencil is symmetric
+    A.mult(u, b)                     # the operator is symmetric (a square grid)
     for g in got:
         np.testing.assert_allclose(g.cpu().numpy(), b.numpy(), rtol=1e-13, atol=1e-13)
 
