@@ -55,6 +55,18 @@ void ensure_device() {
     g_init = true;
 }
 
+// A matrix given to the caller, who may ask for the addresses of its arrays:
+// complete on any stream, and in memory that other processes and devices can
+// be given (rb_common.cuh).
+rb_csr_s* handed_out(rb_csr_s* M) {
+    std::unique_ptr<rb_csr_s> own(M);
+    M->rowptr.to_handle_memory();
+    M->cols.to_handle_memory();
+    M->vals.to_handle_memory();
+    RB_CUDA(cudaStreamSynchronize(stream()));
+    return own.release();
+}
+
 #define NEED(p) RB_REQUIRE((p) != nullptr, #p " is NULL")
 
 }  // namespace
@@ -106,7 +118,11 @@ int rb_csr_create(int n_rows, int n_cols, int64_t nnz, const int* rowptr, const 
         ensure_device();
         NEED(out); NEED(rowptr);
         RB_REQUIRE(nnz == 0 || (cols && vals), "cols/vals are NULL");
-        std::unique_ptr<rb_csr_s> A(new_csr(n_rows, n_cols, nnz));
+        std::unique_ptr<rb_csr_s> A;
+        {
+            HandleMemory scope;
+            A.reset(new_csr(n_rows, n_cols, nnz));
+        }
         auto kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
         if (!on_device) {
             RB_REQUIRE(rowptr[0] == 0 && rowptr[n_rows] == nnz, "rowptr does not span nnz");
@@ -178,8 +194,7 @@ int rb_csr_sort_diag_first(rb_csr A) {
 int rb_csr_transpose(rb_csr A, rb_csr* out) {
     return guarded([&]() -> int {
         NEED(A); NEED(out);
-        *out = transpose(*A);
-        RB_CUDA(cudaStreamSynchronize(stream()));
+        *out = handed_out(transpose(*A));
         return RB_OK;
     });
 }
@@ -192,7 +207,10 @@ int rb_vec_create(int n, rb_vec* out) {
         RB_REQUIRE(n >= 0, "negative vector size");
         auto* v = new rb_vec_s();
         v->n = n;
-        v->v.alloc((size_t)n + 1);
+        {
+            HandleMemory scope;
+            v->v.alloc((size_t)n + 1);
+        }
         v->v.zero();
         *out = v;
         return RB_OK;
@@ -517,7 +535,7 @@ int rb_bsr_spmv_T(rb_bsr A, rb_vec x, rb_vec b) {
 int rb_bsr_to_csr(rb_bsr A, rb_csr* out) {
     return guarded([&]() -> int {
         NEED(A); NEED(out);
-        *out = bsr_to_csr(*A);
+        *out = handed_out(bsr_to_csr(*A));
         return RB_OK;
     });
 }
@@ -555,7 +573,10 @@ int rb_stencil_grid(const double* stencil, const int* grid, int dim, rb_csr* out
     return guarded([&]() -> int {
         ensure_device();
         NEED(stencil); NEED(grid); NEED(out);
-        return rb_stencil_grid_impl(stencil, grid, dim, out);
+        rb_csr A = nullptr;
+        const int rc = rb_stencil_grid_impl(stencil, grid, dim, &A);
+        if (rc == RB_OK) *out = handed_out(A);
+        return rc;
     });
 }
 
@@ -675,8 +696,7 @@ int rb_strength(rb_csr A, int kind, double theta, rb_csr* S) {
     return guarded([&]() -> int {
         NEED(A); NEED(S);
         RB_REQUIRE(kind == RB_STRENGTH_CLASSICAL || kind == RB_STRENGTH_SYMMETRIC, "unknown strength kind");
-        *S = strength(*A, kind, theta);
-        RB_CUDA(cudaStreamSynchronize(stream()));
+        *S = handed_out(strength(*A, kind, theta));
         return RB_OK;
     });
 }
@@ -731,8 +751,7 @@ int rb_interpolation(rb_csr A, rb_csr S, const int* states, int kind, double fil
                    "unknown interpolation kind");
         DevArray<int> st((size_t)std::max(A->n_rows, 1));
         st.upload(states, A->n_rows);
-        *P = interpolation(*A, *S, st.get(), kind, filter);
-        RB_CUDA(cudaStreamSynchronize(stream()));
+        *P = handed_out(interpolation(*A, *S, st.get(), kind, filter));
         return RB_OK;
     });
 }
@@ -781,7 +800,7 @@ int rb_fit_candidates(int n_rows, int n_aggs, const int* aggregates, const doubl
         agg.upload(aggregates, n_rows);
         DevArray<double> Bd((size_t)std::max(n_rows, 1)), Rd((size_t)std::max(n_aggs, 1));
         Bd.upload(B, n_rows);
-        *T = fit_candidates(n_rows, n_aggs, agg.get(), Bd.get(), Rd.get());
+        *T = handed_out(fit_candidates(n_rows, n_aggs, agg.get(), Bd.get(), Rd.get()));
         Rd.download(R, n_aggs);
         RB_CUDA(cudaStreamSynchronize(stream()));
         return RB_OK;
@@ -792,8 +811,7 @@ int rb_jacobi_prolongation(rb_csr A, rb_csr T, double omega, int steps, rb_csr* 
     return guarded([&]() -> int {
         NEED(A); NEED(T); NEED(P);
         RB_REQUIRE(steps >= 0, "steps < 0");
-        *P = jacobi_prolongation(*A, *T, omega, steps);
-        RB_CUDA(cudaStreamSynchronize(stream()));
+        *P = handed_out(jacobi_prolongation(*A, *T, omega, steps));
         return RB_OK;
     });
 }
@@ -801,8 +819,7 @@ int rb_jacobi_prolongation(rb_csr A, rb_csr T, double omega, int steps, rb_csr* 
 int rb_spgemm(rb_csr A, rb_csr B, rb_csr* C) {
     return guarded([&]() -> int {
         NEED(A); NEED(B); NEED(C);
-        *C = spgemm(*A, *B);
-        RB_CUDA(cudaStreamSynchronize(stream()));
+        *C = handed_out(spgemm(*A, *B));
         return RB_OK;
     });
 }
@@ -810,8 +827,7 @@ int rb_spgemm(rb_csr A, rb_csr B, rb_csr* C) {
 int rb_rap(rb_csr A, rb_csr P, int diag_first, rb_csr* Ac) {
     return guarded([&]() -> int {
         NEED(A); NEED(P); NEED(Ac);
-        *Ac = rap(*A, *P, nullptr, diag_first != 0);
-        RB_CUDA(cudaStreamSynchronize(stream()));
+        *Ac = handed_out(rap(*A, *P, nullptr, diag_first != 0));
         return RB_OK;
     });
 }
@@ -913,7 +929,10 @@ int rb_amg_level_matrix(rb_amg ml, int level, int which, rb_csr* out) {
         const MasterLevel& M = ml->h.master[level];
         const rb_csr_s* src = which == 0 ? M.A.get() : which == 1 ? M.P.get() : M.R.get();
         RB_REQUIRE(src != nullptr, "the coarsest level has no P/R");
-        *out = clone_csr(*src);
+        {
+            HandleMemory scope;
+            *out = clone_csr(*src);
+        }
         RB_CUDA(cudaStreamSynchronize(stream()));
         return RB_OK;
     });
@@ -1095,8 +1114,7 @@ int rb_fv_assemble(int nx, int ny, const double* k, rb_csr* A) {
     return guarded([&]() -> int {
         NEED(k); NEED(A);
         ensure_device();
-        *A = fv_assemble(nx, ny, k);
-        RB_CUDA(cudaStreamSynchronize(stream()));
+        *A = handed_out(fv_assemble(nx, ny, k));
         return RB_OK;
     });
 }

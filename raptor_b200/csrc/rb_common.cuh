@@ -64,20 +64,31 @@ int resident_blocks_per_sm(const void* fn, int threads);
 // the library is one); read through rb_device_alloc_count.
 long long& device_alloc_counter();
 
-// Device memory behind DevArray (sparse.cu): stream-ordered allocations from
-// a pool of the library's own, one a device.  *pooled says which kind came
-// back (inside a stream capture it is a plain cudaMalloc, as it would
-// otherwise become a node of the caller's graph).  Everything allocated
-// during a call is used on stream() only, so freeing in stream order is
-// enough for it; memory that a caller may have borrowed (handles) is freed
-// under a HandleRelease, which waits for the device first, as cudaFree does.
-void* device_alloc(size_t bytes, bool* pooled);
-void device_free(void* p, bool pooled) noexcept;
+// Device memory behind DevArray (sparse.cu):
+//   kPool    stream-ordered allocations from a pool of the library's own, one
+//            a device: everything inside a call and inside a handle.
+//   kHandle  arrays whose address a caller can ask for (vectors, and the
+//            matrices handed out), cut from cudaMalloc'd slabs
+//            (handle_heap.cuh): taken while a HandleMemory is in scope.
+//   kDriver  cudaMalloc itself: large arrays, and inside a stream capture
+//            (where the others would become nodes of the caller's graph).
+// What a call allocates for itself is used on stream() only, so freeing it in
+// stream order is enough; what outlives the call that made it is freed under
+// a HandleRelease, which waits for the device first, as cudaFree does.
+enum class Mem : unsigned char { kDriver, kPool, kHandle };
+void* device_alloc(size_t bytes, Mem* kind);
+void device_free(void* p, Mem kind) noexcept;
 struct HandleRelease {
     HandleRelease();
     ~HandleRelease();
     HandleRelease(const HandleRelease&) = delete;
     HandleRelease& operator=(const HandleRelease&) = delete;
+};
+struct HandleMemory {
+    HandleMemory();
+    ~HandleMemory();
+    HandleMemory(const HandleMemory&) = delete;
+    HandleMemory& operator=(const HandleMemory&) = delete;
 };
 
 // A pinned host block of kPinnedBlock bytes, and its return (no copy from or
@@ -91,16 +102,16 @@ template <typename T>
 struct DevArray {
     T* p = nullptr;
     size_t n = 0;
-    bool pooled = false;
+    Mem kind = Mem::kDriver;
     DevArray() = default;
     explicit DevArray(size_t count) { alloc(count); }
     DevArray(const DevArray&) = delete;
     DevArray& operator=(const DevArray&) = delete;
-    DevArray(DevArray&& o) noexcept : p(o.p), n(o.n), pooled(o.pooled) { o.p = nullptr; o.n = 0; }
+    DevArray(DevArray&& o) noexcept : p(o.p), n(o.n), kind(o.kind) { o.p = nullptr; o.n = 0; }
     DevArray& operator=(DevArray&& o) noexcept {
         if (this != &o) {
             release();
-            p = o.p; n = o.n; pooled = o.pooled; o.p = nullptr; o.n = 0;
+            p = o.p; n = o.n; kind = o.kind; o.p = nullptr; o.n = 0;
         }
         return *this;
     }
@@ -108,13 +119,13 @@ struct DevArray {
     void alloc(size_t count) {
         release();
         if (count) {
-            p = static_cast<T*>(::rb::device_alloc(sizeof(T) * count, &pooled));
+            p = static_cast<T*>(::rb::device_alloc(sizeof(T) * count, &kind));
             ++::rb::device_alloc_counter();
         }
         n = count;
     }
     void release() {
-        if (p) ::rb::device_free(p, pooled);
+        if (p) ::rb::device_free(p, kind);
         p = nullptr;
         n = 0;
     }
@@ -132,6 +143,14 @@ struct DevArray {
         download(h.data(), n);
         RB_CUDA(cudaStreamSynchronize(stream()));
         return h;
+    }
+    // Pool memory exchanged for handle memory, with its contents (on stream()).
+    void to_handle_memory() {
+        if (!p || kind != Mem::kPool) return;
+        HandleMemory scope;
+        DevArray<T> h(n);
+        RB_CUDA(cudaMemcpyAsync(h.p, p, sizeof(T) * n, cudaMemcpyDeviceToDevice, stream()));
+        *this = std::move(h);
     }
     T* get() const { return p; }
     size_t size() const { return n; }

@@ -6,6 +6,7 @@
 #include <mutex>
 #include <unordered_map>
 
+#include "handle_heap.cuh"
 #include "rb_internal.cuh"
 #include "spmv.cuh"
 
@@ -61,7 +62,12 @@ constexpr size_t kPoolLargest = (size_t)64 << 20;
 constexpr int kMaxDevices = 64;
 std::mutex g_pool_mu;
 cudaMemPool_t g_pools[kMaxDevices] = {};
-thread_local int t_handle_release = 0;
+thread_local int t_handle_release = 0, t_handle_memory = 0;
+std::mutex g_heap_mu;
+HandleHeap* heaps() {
+    static auto* h = new HandleHeap[kMaxDevices];   // outlives every static handle
+    return h;
+}
 
 cudaMemPool_t pool_of_device() {
     int dev = 0;
@@ -88,39 +94,90 @@ bool capturing(cudaStream_t s) {
 }
 }  // namespace
 
-void* device_alloc(size_t bytes, bool* pooled) {
+namespace {
+// After an allocation failed for want of memory: what the library keeps but
+// does not use goes back to the driver.
+void give_back() {
+    (void)cudaGetLastError();
+    RB_CUDA(cudaDeviceSynchronize());
+    RB_CUDA(cudaMemPoolTrimTo(pool_of_device(), 0));
+    int dev = 0;
+    RB_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(g_heap_mu);
+    heaps()[dev].trim([](char* base) { cudaFree(base); });
+}
+
+void* handle_alloc(size_t bytes) {
+    int dev = 0;
+    RB_CUDA(cudaGetDevice(&dev));
+    RB_REQUIRE(dev >= 0 && dev < kMaxDevices, "device index out of range");
+    auto get = [](size_t size) {
+        void* base = nullptr;
+        RB_CUDA(cudaMalloc(&base, size));
+        return base;
+    };
+    {
+        std::lock_guard<std::mutex> lock(g_heap_mu);
+        try {
+            return heaps()[dev].alloc(bytes, get);
+        } catch (const Error& e) {
+            (void)cudaGetLastError();
+            if (e.code != RB_ERR_OOM) throw;
+        }
+    }
+    give_back();
+    std::lock_guard<std::mutex> lock(g_heap_mu);
+    try {
+        return heaps()[dev].alloc(bytes, get, 0);   // a slab of this block only
+    } catch (...) {
+        (void)cudaGetLastError();
+        throw;
+    }
+}
+}  // namespace
+
+void* device_alloc(size_t bytes, Mem* kind) {
     void* p = nullptr;
     cudaStream_t s = stream();
+    cudaError_t e;
     if (bytes >= kPoolLargest || capturing(s)) {
-        *pooled = false;
-        cudaError_t e = cudaMalloc(&p, bytes);
-        if (e == cudaErrorMemoryAllocation && !capturing(s)) {   // what the pool keeps may be what is missing
-            (void)cudaGetLastError();
-            RB_CUDA(cudaDeviceSynchronize());
-            RB_CUDA(cudaMemPoolTrimTo(pool_of_device(), 0));
+        *kind = Mem::kDriver;
+        e = cudaMalloc(&p, bytes);
+        if (e == cudaErrorMemoryAllocation && !capturing(s)) {   // what is kept may be what is missing
+            give_back();
             e = cudaMalloc(&p, bytes);
         }
-        if (e != cudaSuccess) (void)cudaGetLastError();
-        RB_CUDA(e);
-        return p;
-    }
-    *pooled = true;
-    cudaMemPool_t pool = pool_of_device();
-    cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, s);
-    if (e == cudaErrorMemoryAllocation) {
-        (void)cudaGetLastError();
-        RB_CUDA(cudaDeviceSynchronize());
-        RB_CUDA(cudaMemPoolTrimTo(pool, 0));
+    } else if (t_handle_memory > 0) {
+        *kind = Mem::kHandle;
+        return handle_alloc(bytes);
+    } else {
+        *kind = Mem::kPool;
+        cudaMemPool_t pool = pool_of_device();
         e = cudaMallocFromPoolAsync(&p, bytes, pool, s);
+        if (e == cudaErrorMemoryAllocation) {
+            give_back();
+            e = cudaMallocFromPoolAsync(&p, bytes, pool, s);
+        }
     }
     if (e != cudaSuccess) (void)cudaGetLastError();
     RB_CUDA(e);
     return p;
 }
 
-void device_free(void* p, bool pooled) noexcept {
+void device_free(void* p, Mem kind) noexcept {
+    const bool pooled = kind == Mem::kPool;
     cudaError_t e = cudaErrorUnknown;
-    if (!pooled) {
+    if (kind == Mem::kHandle) {
+        if (t_handle_release == 0 && cudaDeviceSynchronize() != cudaSuccess) (void)cudaGetLastError();
+        std::lock_guard<std::mutex> lock(g_heap_mu);
+        for (int d = 0; d < kMaxDevices; d++)
+            if (heaps()[d].owns(p)) {
+                heaps()[d].free(p, [](char* base) { cudaFree(base); });
+                break;
+            }
+        return;
+    }
+    if (kind == Mem::kDriver) {
         e = cudaFree(p);
     } else if (t_handle_release > 0) {
         // the device is idle (HandleRelease); a stream the caller set may be
@@ -144,6 +201,9 @@ HandleRelease::HandleRelease() {
     ++t_handle_release;
 }
 HandleRelease::~HandleRelease() { --t_handle_release; }
+
+HandleMemory::HandleMemory() { ++t_handle_memory; }
+HandleMemory::~HandleMemory() { --t_handle_memory; }
 
 // Small pinned staging blocks (device scalars read back): cudaMallocHost
 // takes over a millisecond, as long as a small setup's kernels, so freed

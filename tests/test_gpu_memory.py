@@ -1,6 +1,7 @@
 """Device memory of the library: freed memory is kept for the next allocation
 up to a bound, and memory a caller borrowed from a handle is not handed to
 anyone else before the caller's pending work on it is done."""
+import ctypes
 import gc
 
 import numpy as np
@@ -32,6 +33,44 @@ def test_freed_memory_is_given_back_above_the_bound(log2n, kept):
     rb.synchronize()
     # (and the driver's own granularity)
     assert torch.cuda.mem_get_info()[0] > before - kept - (256 << 20)
+
+
+def _ipc_capable(ptr):
+    """Whether cudaIpcGetMemHandle takes the address (a query only)."""
+    from cuda.bindings import driver
+
+    attr = driver.CUpointer_attribute.CU_POINTER_ATTRIBUTE_IS_LEGACY_CUDA_IPC_CAPABLE
+    err, capable = driver.cuPointerGetAttribute(attr, int(ptr))
+    assert err == driver.CUresult.CUDA_SUCCESS, err
+    return bool(capable)
+
+
+def test_addresses_given_out_can_be_shared_between_processes():
+    """Vectors and matrices of every origin and of sizes on both sides of the
+    pool's and the slabs' limits lie in memory of cudaMalloc, which other
+    processes (CUDA IPC) and other devices (peer access) can be given."""
+    for n in (1, 31, 1000, 1 << 16, (1 << 22) - 1, 1 << 22, 1 << 23):
+        assert _ipc_capable(rb.ParVector(n).device_ptr()), n
+    A = rb.par_stencil_grid(rb.diffusion_stencil_2d(0.1, 0.4), [40, 40])
+    n = A.global_num_rows
+    S = A.strength(rb.Classical, 0.25)
+    ml = rb.ParRugeStubenSolver(0.25, rb.PMIS, rb.ModClassical, rb.Classical, rb.Jacobi)
+    ml.setup(A)
+    blocks = rb.BSRMatrix.from_arrays(1, 1, 2, 2, [0, 1], [0], np.arange(1.0, 5.0).reshape(1, 2, 2))
+    mats = {"grid": A, "strength": S, "transpose": A.transpose(), "product": A.mult_matrix(A),
+            "level A": ml.level_matrix(1, "A"), "level P": ml.level_matrix(0, "P"),
+            "blocks": blocks.to_CSR(),
+            "arrays": rb.ParCSRMatrix.from_arrays(2, 2, [0, 1, 2], [0, 1], [1.0, 2.0])}
+    for name, M in mats.items():
+        ptrs = [ctypes.c_void_p() for _ in range(3)]
+        rb.check(rb.lib().rb_csr_device_arrays(M.h, *map(ctypes.byref, ptrs)))
+        for ptr in ptrs:
+            assert _ipc_capable(ptr.value), name
+    x = rb.ParVector(n, values=np.ones(n))
+    y, z = rb.ParVector(n), rb.ParVector(n)
+    A.mult(x, y)
+    mats["transpose"].mult(x, z)     # (the square grid's operator is symmetric)
+    np.testing.assert_allclose(y.numpy(), z.numpy(), rtol=0, atol=1e-13)
 
 
 def test_borrowed_memory_outlives_pending_reads():
