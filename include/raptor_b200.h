@@ -97,7 +97,7 @@ int rb_bsr_spmv_T(rb_bsr A, rb_vec x, rb_vec b);
 int rb_bsr_to_csr(rb_bsr A, rb_csr* out);
 
 /* ParVector (core/par_vector.hpp:44-176) */
-int rb_vec_create(int n, rb_vec* out);
+int rb_vec_create(int n, rb_vec* out);            /* zeros, there on return for any stream */
 int rb_vec_destroy(rb_vec v);
 int rb_vec_size(rb_vec v, int* n);
 int rb_vec_upload(rb_vec v, const double* host);   /* host or device source */

@@ -205,14 +205,17 @@ int rb_vec_create(int n, rb_vec* out) {
         ensure_device();
         NEED(out);
         RB_REQUIRE(n >= 0, "negative vector size");
-        auto* v = new rb_vec_s();
+        std::unique_ptr<rb_vec_s> v(new rb_vec_s());
         v->n = n;
         {
             HandleMemory scope;
             v->v.alloc((size_t)n + 1);
         }
         v->v.zero();
-        *out = v;
+        // the zeros are there on return: the caller may write on any stream
+        // (in a capture they are a node of the caller's graph)
+        if (!capturing(stream())) RB_CUDA(cudaStreamSynchronize(stream()));
+        *out = v.release();
         return RB_OK;
     });
 }

@@ -64,6 +64,9 @@ int resident_blocks_per_sm(const void* fn, int threads);
 // the library is one); read through rb_device_alloc_count.
 long long& device_alloc_counter();
 
+// Whether a capture of s is in progress.
+bool capturing(cudaStream_t s);
+
 // Device memory behind DevArray (sparse.cu):
 //   kPool    stream-ordered allocations from a pool of the library's own, one
 //            a device: everything inside a call and inside a handle.

@@ -87,12 +87,12 @@ cudaMemPool_t pool_of_device() {
     }
     return g_pools[dev];
 }
+}  // namespace
 
 bool capturing(cudaStream_t s) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
 }
-}  // namespace
 
 namespace {
 // After an allocation failed for want of memory: what the library keeps but

@@ -73,6 +73,35 @@ def test_addresses_given_out_can_be_shared_between_processes():
     np.testing.assert_allclose(y.numpy(), z.numpy(), rtol=0, atol=1e-13)
 
 
+def test_a_new_vector_may_be_written_on_any_stream():
+    """With work queued on the library's stream, a vector is created and at
+    once filled through its view on another stream: its zeros are in place
+    by then."""
+    s, mine = torch.cuda.Stream(), torch.cuda.Stream()
+    busy = torch.zeros(1 << 26, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    vs = []
+    try:
+        rb.set_stream(s.cuda_stream)
+        for n in (5, 1 << 16, 1 << 22):
+            with torch.cuda.stream(s):
+                for _ in range(20):
+                    busy += 1.0
+            v = rb.ParVector(n)
+            assert s.query()
+            with torch.cuda.stream(mine):
+                v.torch_view().fill_(3.0)
+            vs.append(v)
+        mine.synchronize()
+        s.synchronize()
+        for v in vs:
+            assert torch.all(v.torch_view() == 3.0)
+            assert v.inner_product(v) == 9.0 * v.local_n
+    finally:
+        rb.synchronize()
+        rb.set_stream(0)
+
+
 def test_borrowed_memory_outlives_pending_reads():
     n = 1 << 22
     for rep in range(5):
