@@ -212,8 +212,11 @@ int adjoint_solve(const rb_csr_s& A, Hierarchy& H, double* lambda, const double*
     if (H.adj_A != &A) {
         H.adj_sym = is_symmetric(A, 1e-14);
         H.adj_A = &A;
-        H.adj.reset();
-        H.adj_AT.reset();
+        if (H.adj) {
+            HandleRelease idle;
+            H.adj.reset();
+            H.adj_AT.reset();
+        }
     }
     RB_CUDA(cudaMemsetAsync(lambda, 0, sizeof(double) * n, stream()));
     int rc, nh = 0;

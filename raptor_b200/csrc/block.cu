@@ -370,8 +370,12 @@ void block_residual64(BlockState& bs, const rb_csr_s& A, const double* X, const 
 BlockState& Hierarchy::block_state(int k) {
     RB_REQUIRE(k >= 2 && k <= kMaxBlockK, "block: k must be in 2..32");
     if (blk && blk->k == k) return *blk;
+    if (blk) {   // cycles of the other k may be pending, on another stream too
+        HandleRelease idle;
+        release_graphs();
+        blk.reset();
+    }
     release_graphs();
-    blk.reset();
     auto s = std::make_shared<BlockState>();
     s->k = k;
     const long n = master[0].A->n_rows;

@@ -186,7 +186,10 @@ int rb_csr_sort_diag_first(rb_csr A) {
         NEED(A);
         sort_rows_diag_first(*A, true);
         RB_CHECK_LAUNCH();
-        A->tmap.reset();  // entry positions moved
+        if (A->tmap) {   // entry positions moved; products on any stream may be reading it
+            HandleRelease idle;
+            A->tmap.reset();
+        }
         return RB_OK;
     });
 }

@@ -76,8 +76,9 @@ bool capturing(cudaStream_t s);
 //   kDriver  cudaMalloc itself: large arrays, and inside a stream capture
 //            (where the others would become nodes of the caller's graph).
 // What a call allocates for itself is used on stream() only, so freeing it in
-// stream order is enough; what outlives the call that made it is freed under
-// a HandleRelease, which waits for the device first, as cudaFree does.
+// stream order is enough; what outlives the call that made it (a handle, a
+// handle's workspaces and maps) is freed under a HandleRelease, which waits
+// for the device first, as cudaFree does.
 enum class Mem : unsigned char { kDriver, kPool, kHandle };
 void* device_alloc(size_t bytes, Mem* kind);
 void device_free(void* p, Mem kind) noexcept;

@@ -184,12 +184,15 @@ void device_free(void* p, Mem kind) noexcept {
         // gone by now, so the library's own orders the free
         if (g_own_stream || cudaStreamCreateWithFlags(&g_own_stream, cudaStreamNonBlocking) == cudaSuccess)
             e = cudaFreeAsync(p, g_own_stream);
-    } else if (g_stream && !capturing(g_stream)) {
-        e = cudaFreeAsync(p, g_stream);
+    } else {
+        const cudaStream_t s = g_stream ? g_stream : g_own_stream;
+        if (s && !capturing(s)) e = cudaFreeAsync(p, s);
     }
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
-        if (pooled) cudaFree(p);
+        // (cudaFree does not wait for a pool's memory; where waiting is
+        // refused, as in a capture, the memory stays allocated)
+        if (pooled && cudaDeviceSynchronize() == cudaSuccess) cudaFree(p);
         (void)cudaGetLastError();
     }
 }

@@ -102,6 +102,42 @@ def test_a_new_vector_may_be_written_on_any_stream():
         rb.set_stream(0)
 
 
+def test_workspaces_replaced_while_another_stream_uses_them():
+    """A block cycle of 4 columns is pending on one stream when one of 8
+    columns on another replaces the hierarchy's workspaces."""
+    A = rb.par_stencil_grid(rb.diffusion_stencil_2d(0.1, 0.4), [300, 300])
+    n = A.global_num_rows
+    ml = rb.ParRugeStubenSolver(0.25, rb.PMIS, rb.Extended, rb.Classical, rb.L1Jacobi)
+    ml.setup(A)
+    rng = np.random.default_rng(8)
+    B = {k: rb.ParVector(n * k, values=rng.uniform(-1, 1, n * k)) for k in (4, 8)}
+    want = {}
+    for k in (8, 4):
+        X = rb.ParVector(n * k)
+        ml.cycle_block(X, B[k], k)
+        want[k] = X.numpy()
+    X = {k: rb.ParVector(n * k) for k in (4, 8)}
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    busy = torch.zeros(1 << 26, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    try:
+        rb.set_stream(first.cuda_stream)
+        with torch.cuda.stream(first):
+            for _ in range(20):
+                busy += 1.0
+        ml.cycle_block(X[4], B[4], 4)
+        rb.set_stream(second.cuda_stream)
+        ml.cycle_block(X[8], B[8], 8)
+        assert first.query()          # nothing is freed under a pending cycle
+        first.synchronize()
+        second.synchronize()
+    finally:
+        rb.synchronize()
+        rb.set_stream(0)
+    for k in (4, 8):
+        np.testing.assert_allclose(X[k].numpy(), want[k], rtol=1e-12, atol=1e-14)
+
+
 def test_borrowed_memory_outlives_pending_reads():
     n = 1 << 22
     for rep in range(5):
