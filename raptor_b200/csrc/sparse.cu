@@ -739,8 +739,10 @@ struct ReduceScratch {
     std::once_flag once;
 };
 ReduceScratch& scratch() {
-    static ReduceScratch s;
-    return s;
+    // (never destroyed: at process exit the stream its frees would be ordered
+    // on may be one of the caller's that is gone)
+    static auto* s = new ReduceScratch();
+    return *s;
 }
 }  // namespace
 

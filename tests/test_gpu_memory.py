@@ -3,6 +3,9 @@ up to a bound, and memory a caller borrowed from a handle is not handed to
 anyone else before the caller's pending work on it is done."""
 import ctypes
 import gc
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -136,6 +139,27 @@ def test_workspaces_replaced_while_another_stream_uses_them():
         rb.set_stream(0)
     for k in (4, 8):
         np.testing.assert_allclose(X[k].numpy(), want[k], rtol=1e-12, atol=1e-14)
+
+
+def test_process_exit_after_the_callers_stream_is_gone():
+    code = """
+import torch, raptor_b200 as rb
+from cuda.bindings import runtime
+rb.init(0)
+err, s = runtime.cudaStreamCreate()
+rb.set_stream(int(s))
+x = rb.ParVector(1000)
+x.set_const_value(2.0)
+assert x.norm() == 2.0 * 1000 ** 0.5
+rb.synchronize()
+del x
+(err,) = runtime.cudaStreamDestroy(s)
+assert int(err) == 0
+print("ended", flush=True)
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0 and r.stdout.strip() == "ended", r.stderr
 
 
 def test_borrowed_memory_outlives_pending_reads():
