@@ -45,6 +45,11 @@ int rb_init(int device);
 int rb_set_stream(void* cuda_stream);
 /* Wait for all work queued on the library stream. */
 int rb_synchronize(void);
+/* Give device memory that the library keeps for its next allocations (at most
+ * 2 GiB of temporaries and 1 GiB of vectors and matrices while handles are
+ * alive, 384 MiB once all are destroyed) back to the driver, for another
+ * allocator in the process.  Waits for the device. */
+int rb_trim(void);
 /* Library version string. */
 const char* rb_version(void);
 

@@ -928,6 +928,12 @@ def synchronize():
     check(lib().rb_synchronize())
 
 
+def trim():
+    """Give device memory that the library keeps for its next allocations
+    back to the driver."""
+    check(lib().rb_trim())
+
+
 def version():
     return lib().rb_version().decode()
 

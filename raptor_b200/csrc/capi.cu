@@ -111,6 +111,14 @@ int rb_synchronize(void) {
     });
 }
 
+int rb_trim(void) {
+    return guarded([&]() -> int {
+        ensure_device();
+        trim_memory();
+        return RB_OK;
+    });
+}
+
 // ------------------------------------------------------------ containers --
 int rb_csr_create(int n_rows, int n_cols, int64_t nnz, const int* rowptr, const int* cols,
                   const double* vals, int on_device, rb_csr* out) {

@@ -84,10 +84,10 @@ public:
         if (idle_ > kKeep) trim(put);
     }
 
-    // Gives every idle slab back.
+    // Gives idle slabs back until at most `keep` bytes of them are left.
     template <class Put>
-    void trim(Put&& put) {
-        for (auto s = slabs_.begin(); s != slabs_.end();) {
+    void trim(Put&& put, size_t keep = 0) {
+        for (auto s = slabs_.begin(); s != slabs_.end() && idle_ > keep;) {
             auto f = free_.find(s->first);
             if (f != free_.end() && f->second == s->second) {
                 char* base = s->first;

@@ -82,6 +82,8 @@ bool capturing(cudaStream_t s);
 enum class Mem : unsigned char { kDriver, kPool, kHandle };
 void* device_alloc(size_t bytes, Mem* kind);
 void device_free(void* p, Mem kind) noexcept;
+// Gives the memory that is kept but not in use back to the driver.
+void trim_memory();
 struct HandleRelease {
     HandleRelease();
     ~HandleRelease();

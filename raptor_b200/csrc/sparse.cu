@@ -2,6 +2,7 @@
 // deterministic reductions and the FP64 SpMV primitives of the C ABI.
 #include <cub/cub.cuh>
 
+#include <atomic>
 #include <climits>
 #include <mutex>
 #include <unordered_map>
@@ -52,17 +53,23 @@ void set_stream(cudaStream_t s) { g_stream = s ? s : nullptr; }
 // adjoint solve 37.0 -> 14.0 ms).  The pool keeps at most kPoolKeep bytes
 // of freed memory: the driver gives back what is above at every
 // synchronisation, and an allocation that fails gives back the rest and
-// tries once more.  Arrays of kPoolLargest and more stay with cudaMalloc:
+// tries once more; once the last array is freed all but kIdleKeep goes back,
+// and rb_trim gives back whatever is not in use (not all of it at once: a
+// differentiated solve makes and frees all its handles in every step, 37 ms
+// with nothing kept).  Arrays of kPoolLargest and more stay with cudaMalloc:
 // pooled, the gigabytes a large hierarchy frees are unmapped at the next
 // synchronisation, wherever it falls (a 192^3 setup 700 -> 1720 ms and the
 // first solve after it 10.8 -> 380 ms; with the limit 606 ms and as before).
 namespace {
 constexpr unsigned long long kPoolKeep = 2ull << 30;
 constexpr size_t kPoolLargest = (size_t)64 << 20;
+constexpr size_t kIdleKeep = (size_t)256 << 20;     // of the pool with no array left
+constexpr size_t kIdleSlabs = (size_t)128 << 20;    // of the handles' slabs then
 constexpr int kMaxDevices = 64;
 std::mutex g_pool_mu;
 cudaMemPool_t g_pools[kMaxDevices] = {};
 thread_local int t_handle_release = 0, t_handle_memory = 0;
+std::atomic<long long> g_live{0};   // arrays of DevArrays
 std::mutex g_heap_mu;
 HandleHeap* heaps() {
     static auto* h = new HandleHeap[kMaxDevices];   // outlives every static handle
@@ -95,16 +102,16 @@ bool capturing(cudaStream_t s) {
 }
 
 namespace {
-// After an allocation failed for want of memory: what the library keeps but
-// does not use goes back to the driver.
-void give_back() {
+// What the library keeps but does not use goes back to the driver, but for
+// some bytes of the pool and of the slabs.
+void give_back(size_t keep_pool, size_t keep_slabs) {
     (void)cudaGetLastError();
     RB_CUDA(cudaDeviceSynchronize());
-    RB_CUDA(cudaMemPoolTrimTo(pool_of_device(), 0));
+    RB_CUDA(cudaMemPoolTrimTo(pool_of_device(), keep_pool));
     int dev = 0;
     RB_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lock(g_heap_mu);
-    heaps()[dev].trim([](char* base) { cudaFree(base); });
+    heaps()[dev].trim([](char* base) { cudaFree(base); }, keep_slabs);
 }
 
 void* handle_alloc(size_t bytes) {
@@ -125,7 +132,7 @@ void* handle_alloc(size_t bytes) {
             if (e.code != RB_ERR_OOM) throw;
         }
     }
-    give_back();
+    give_back(0, 0);
     std::lock_guard<std::mutex> lock(g_heap_mu);
     try {
         return heaps()[dev].alloc(bytes, get, 0);   // a slab of this block only
@@ -136,6 +143,8 @@ void* handle_alloc(size_t bytes) {
 }
 }  // namespace
 
+void trim_memory() { give_back(0, 0); }
+
 void* device_alloc(size_t bytes, Mem* kind) {
     void* p = nullptr;
     cudaStream_t s = stream();
@@ -144,29 +153,33 @@ void* device_alloc(size_t bytes, Mem* kind) {
         *kind = Mem::kDriver;
         e = cudaMalloc(&p, bytes);
         if (e == cudaErrorMemoryAllocation && !capturing(s)) {   // what is kept may be what is missing
-            give_back();
+            give_back(0, 0);
             e = cudaMalloc(&p, bytes);
         }
     } else if (t_handle_memory > 0) {
         *kind = Mem::kHandle;
-        return handle_alloc(bytes);
+        p = handle_alloc(bytes);
+        ++g_live;
+        return p;
     } else {
         *kind = Mem::kPool;
         cudaMemPool_t pool = pool_of_device();
         e = cudaMallocFromPoolAsync(&p, bytes, pool, s);
         if (e == cudaErrorMemoryAllocation) {
-            give_back();
+            give_back(0, 0);
             e = cudaMallocFromPoolAsync(&p, bytes, pool, s);
         }
     }
     if (e != cudaSuccess) (void)cudaGetLastError();
     RB_CUDA(e);
+    ++g_live;
     return p;
 }
 
 void device_free(void* p, Mem kind) noexcept {
     const bool pooled = kind == Mem::kPool;
     cudaError_t e = cudaErrorUnknown;
+    --g_live;
     if (kind == Mem::kHandle) {
         if (t_handle_release == 0 && cudaDeviceSynchronize() != cudaSuccess) (void)cudaGetLastError();
         std::lock_guard<std::mutex> lock(g_heap_mu);
@@ -203,7 +216,14 @@ HandleRelease::HandleRelease() {
     if (t_handle_release == 0 && cudaDeviceSynchronize() != cudaSuccess) (void)cudaGetLastError();
     ++t_handle_release;
 }
-HandleRelease::~HandleRelease() { --t_handle_release; }
+HandleRelease::~HandleRelease() {
+    if (--t_handle_release > 0 || g_live != 0) return;
+    try {
+        give_back(kIdleKeep, kIdleSlabs);
+    } catch (const std::exception&) {   // no device any more, at process exit
+        (void)cudaGetLastError();
+    }
+}
 
 HandleMemory::HandleMemory() { ++t_handle_memory; }
 HandleMemory::~HandleMemory() { --t_handle_memory; }
@@ -260,14 +280,14 @@ int sm_count() {
 void tune_cold_l2(const void* warm, size_t bytes) {
     // 192 MB, above the 126 MB L2; allocated once and kept for the process
     constexpr size_t kFlush = (size_t)192 << 20;
-    static DevArray<char>* buf = nullptr;
+    static void* buf = nullptr;
     if (!buf) {
-        buf = new DevArray<char>();
-        buf->alloc(kFlush);
+        RB_CUDA(cudaMalloc(&buf, kFlush));
+        ++device_alloc_counter();
     }
-    RB_CUDA(cudaMemsetAsync(buf->get(), 0, kFlush, stream()));
+    RB_CUDA(cudaMemsetAsync(buf, 0, kFlush, stream()));
     if (warm && bytes)
-        RB_CUDA(cudaMemcpyAsync(buf->get(), warm, bytes < kFlush ? bytes : kFlush,
+        RB_CUDA(cudaMemcpyAsync(buf, warm, bytes < kFlush ? bytes : kFlush,
                                 cudaMemcpyDeviceToDevice, stream()));
 }
 
@@ -733,17 +753,11 @@ __global__ void __launch_bounds__(256) k_dot(const double* __restrict__ a,
 }
 
 namespace {
+// (memory of the process: never freed, and no array of a handle or a call)
 struct ReduceScratch {
-    DevArray<double> partials;
-    DevArray<unsigned> ticket;
-    std::once_flag once;
-};
-ReduceScratch& scratch() {
-    // (never destroyed: at process exit the stream its frees would be ordered
-    // on may be one of the caller's that is gone)
-    static auto* s = new ReduceScratch();
-    return *s;
-}
+    double* partials = nullptr;
+    unsigned* ticket = nullptr;
+} g_scratch;
 }  // namespace
 
 // One scratch for every reduction on the library stream.  It is allocated
@@ -751,15 +765,16 @@ ReduceScratch& scratch() {
 constexpr int kMaxReduceGrid = 1 << 16;
 
 ReduceSlot global_reduce_slot(int grid) {
-    auto& s = scratch();
+    auto& s = g_scratch;
     RB_REQUIRE(grid <= kMaxReduceGrid, "reduction grid too large");
-    if (!s.partials.size()) {
-        s.partials.alloc(kMaxReduceGrid);
-        s.ticket.alloc(1);
-        s.ticket.zero();
+    if (!s.partials) {
+        RB_CUDA(cudaMalloc(&s.ticket, 256 + sizeof(double) * kMaxReduceGrid));
+        RB_CUDA(cudaMemsetAsync(s.ticket, 0, sizeof(unsigned), stream()));
         RB_CUDA(cudaStreamSynchronize(stream()));
+        s.partials = reinterpret_cast<double*>(reinterpret_cast<char*>(s.ticket) + 256);
+        ++device_alloc_counter();
     }
-    return ReduceSlot{s.partials.get(), s.ticket.get()};
+    return ReduceSlot{s.partials, s.ticket};
 }
 
 void dot_async(const double* a, const double* b, int n, double* result_dev) {

@@ -141,6 +141,47 @@ def test_workspaces_replaced_while_another_stream_uses_them():
         np.testing.assert_allclose(X[k].numpy(), want[k], rtol=1e-12, atol=1e-14)
 
 
+def test_memory_goes_back_once_the_last_handle_is_gone():
+    """A hierarchy and vectors of 1.5 GiB: with every handle destroyed at most
+    384 MiB stay with the library, and after rb.trim() nothing but the
+    driver's granularity (and the two buffers of the process, made by a first
+    small run)."""
+    code = """
+import gc, torch, raptor_b200 as rb
+rb.init(0)
+free = lambda: torch.cuda.mem_get_info()[0]
+def work(m, count):
+    A = rb.par_stencil_grid(rb.laplace_stencil_27pt(), [m, m, m])
+    ml = rb.ParRugeStubenSolver(0.25, rb.PMIS, rb.Extended, rb.Classical, rb.L1Jacobi)
+    ml.setup(A)
+    x, b = rb.ParVector(m ** 3), rb.ParVector(m ** 3)
+    b.set_const_value(1.0)
+    ml.cycle(x, b)
+    many = [rb.ParVector(1 << 21) for _ in range(count)]   # 16 MiB each
+    rb.synchronize()
+    return free()
+work(30, 1)
+gc.collect()
+rb.trim()
+before = free()
+held = work(64, 64)
+assert held < before - (1200 << 20), (before, held)
+gc.collect()
+kept = before - free()
+rb.trim()
+left = before - free()
+print(kept >> 20, left >> 20, flush=True)
+assert kept <= (384 + 64) << 20, kept
+assert left <= 64 << 20, left
+x = rb.ParVector(1 << 21)
+x.set_const_value(1.0)
+assert abs(x.norm() - (1 << 21) ** 0.5) < 1e-9
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
 def test_process_exit_after_the_callers_stream_is_gone():
     code = """
 import torch, raptor_b200 as rb
