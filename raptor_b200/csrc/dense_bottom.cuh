@@ -44,9 +44,10 @@ __device__ __forceinline__ double dense_row(int n, int ld, const double* __restr
     double s = 0.0;
 #pragma unroll 4
     for (int j = (threadIdx.x & 31) * 2; j < ld; j += 64) {
-        const double2 a = __ldg(reinterpret_cast<const double2*>(r + j));
-        s += a.x * (double)__ldg(b + j);
-        s += a.y * (j + 1 < n ? (double)__ldg(b + j + 1) : 0.0);
+        double a[2];
+        *reinterpret_cast<uint4*>(a) = __ldg(reinterpret_cast<const uint4*>(r + j));
+#pragma unroll
+        for (int v = 0; v < 2; v++) s += a[v] * (j + v < n ? (double)__ldg(b + j + v) : 0.0);
     }
     return warp_sum(s);
 }
