@@ -171,11 +171,20 @@ std::string tune_key(const char* op, long n, long long nnz, int vbytes) {
     return b;
 }
 
-// Operators of fewer rows are not timed: every schedule takes the 2 to 3 us of
-// a launch there, so the timing picked one at random -- and with it the order
-// of its sums, which a long CG history at 1e-10 shows (100^2) -- for a
-// first setup longer by its launches.
+// Operators of few rows and few entries take their lanes, index width and
+// storage from size rules and are not timed: every schedule takes the 2 to 3
+// us of a launch there, so the timing picked one at random -- and with it the
+// order of its sums, which a long CG history at 1e-10 shows (100^2) -- for a
+// first setup longer by its launches.  Both limits matter: cycles whose level
+// has 6101 rows of 43 entries (FP64, 3.2 MB) or 11006 of 25 take the same time
+// either way, but with 14401 rows of 45 timing gains 68 -> 63 us (FP64, 7.7
+// MB) and 51 -> 47 (FP32, 5.2 MB), with 14426 of 55 43 -> 41.
 constexpr int kTuneRows = 16384;
+constexpr int kTuneMinRows = 4096;
+constexpr long long kTuneBytes = 4 << 20;
+static bool too_small_to_time(long n, long long nnz, int vbytes) {
+    return n < kTuneMinRows || (n < kTuneRows && nnz * (4 + vbytes) <= kTuneBytes);
+}
 
 // Time the row kernel for each group width and keep the fastest.
 template <typename T>
@@ -185,7 +194,7 @@ static int autotune_group_timed(const CsrView<T>& M, T* xin, T* yout, bool strid
 template <typename T>
 static int autotune_group(const CsrView<T>& M, T* xin, T* yout, const char* op = "rows",
                           bool strided = false) {
-    if (M.n_rows < kTuneRows) return pick_group(M.n_rows, M.nnz);
+    if (too_small_to_time(M.n_rows, M.nnz, (int)sizeof(T))) return pick_group(M.n_rows, M.nnz);
     const std::string key = tune_key((strided ? std::string("s") + op : std::string(op)).c_str(),
                                      M.n_rows, M.nnz, (int)sizeof(T));
     auto& c = tune_cache();
@@ -225,7 +234,7 @@ static void tune_idx16(const CsrView<T>& M, Idx16& I, int G, const T* xin, T* yo
     // the rows allow it (any size), unset lets the timing decide
     const char* env = getenv("RAPTOR_B200_IDX16");
     const int force = (env && env[0] == '0') ? 0 : (env && env[0] == '1') ? 1 : -1;
-    if (force == 0 || M.nnz == 0 || (force < 0 && M.n_rows < kTuneRows)) return;
+    if (force == 0 || M.nnz == 0 || (force < 0 && too_small_to_time(M.n_rows, M.nnz, (int)sizeof(T)))) return;
     const std::string key = tune_key(op, M.n_rows, M.nnz, (int)sizeof(T));
     auto& c = tune_cache();
     auto it = c.m.find(key);
@@ -285,7 +294,7 @@ static int tune_tiles(const CsrView<T>& M, Idx16& I, int G, const T* xin, T* you
     I.tchunks = 0;
     const char* env = getenv("RAPTOR_B200_TILED");
     const int force = (env && env[0] == '0') ? 0 : (env && env[0] == '1') ? 1 : -1;
-    if (force == 0 || M.nnz == 0 || (force < 0 && M.n_rows < kTuneRows)) return G;
+    if (force == 0 || M.nnz == 0 || (force < 0 && too_small_to_time(M.n_rows, M.nnz, (int)sizeof(T)))) return G;
     const std::string key = tune_key(op, M.n_rows, M.nnz, (int)sizeof(T));
     auto& c = tune_cache();
     auto it = c.m.find(key);
@@ -812,7 +821,7 @@ void Hierarchy::build_levels(std::vector<Level<T>>& lv) {
             const std::string key = tune_key("A_dia", V.n, V.A.nnz, (int)sizeof(T));
             auto& c = tune_cache();
             auto it = c.m.find(key);
-            if (V.n < kTuneRows) {
+            if (too_small_to_time(V.n, V.A.nnz, (int)sizeof(T))) {
                 V.dia = true;
             } else if (it != c.m.end()) {
                 V.dia = it->second != 0;
