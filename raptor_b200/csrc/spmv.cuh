@@ -139,7 +139,7 @@ struct EpiResidual {
     __device__ void operator()(long i, A s, double&) const { r[i] = (TY)((A)b[i] - s); }
     // the same, split: operands loaded with the row's own loads, then applied
     struct Pre { TB b; };
-    __device__ Pre pre(long i) const { return Pre{__ldg(b + i)}; }
+    __device__ Pre pre(long i) const { return Pre{b[i]}; }   // (r may be b: not the read-only path)
     template <typename A>
     __device__ void post(long i, A s, double&, const Pre& p) const { r[i] = (TY)((A)p.b - s); }
 };

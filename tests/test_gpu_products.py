@@ -44,6 +44,9 @@ def test_products_with_long_rows_and_columns(n, m, mean, special):
     A.residual(x, u, r)
     A.mult_append(x, a)
     A.mult_T(u, t)
+    own = rb.ParVector(n, values=uh)
+    A.residual(x, own, own)          # in place
+    np.testing.assert_array_equal(own.numpy(), r.numpy())
     want = np.bincount(rows, vals * xh[cols], n)
     wantT = np.bincount(cols, vals * uh[rows], m)
     # |sum error| <= (terms) eps sum |terms|, for any order of the sum
