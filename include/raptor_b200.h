@@ -350,13 +350,18 @@ int rb_amg_level_storage(rb_amg ml, int level, int* ndiag);
  * counterpart in the reference. */
 int rb_amg_level_const_coef(rb_amg ml, int level, int* constant);
 /* 1 when level l's first sweep from zero runs fused with its residual (one
- * pass over A_l; the autotuner's pick), else 0.  No counterpart in the
+ * pass over A_l), else 0.  Timed at level 0 only: below it the restriction
+ * from above writes the first sweep with its right-hand side (0 there, unless
+ * RAPTOR_B200_FUSE_FIRST=1 asked for the fused pass).  No counterpart in the
  * reference. */
 int rb_amg_level_fused_first(rb_amg ml, int level, int* fused);
 /* The level from which the rest of the cycle runs as one cluster launch
  * (-1: none) and the CTAs of that cluster.  No counterpart in the
  * reference (it describes how this library schedules the cycle). */
 int rb_amg_tail_info(rb_amg ml, int* start_level, int* ctas);
+/* The level from which the rest of the cycle is one dense product (-1: none)
+ * and the rows of that level.  No counterpart in the reference. */
+int rb_amg_dense_info(rb_amg ml, int* start_level, int* rows);
 /* The cycle times (ms) the setup measured to pick that level: without the
  * cluster tail first, then for each qualifying start from the coarsest
  * upwards (empty when the choice came from the tune cache or was forced).
@@ -365,9 +370,9 @@ int rb_amg_tail_timings(rb_amg ml, double* ms, int cap, int* count);
 /* Kernels this library has launched so far (graph replays count their
  * kernel nodes). */
 int rb_launch_count(int64_t* count);
-/* Device allocations (cudaMalloc) this library has made so far.  No
- * counterpart in the reference; a diagnostic for callers that audit
- * allocation-free paths. */
+/* Device arrays this library has allocated so far, from the driver, its pool
+ * or its slabs.  No counterpart in the reference; a diagnostic for callers
+ * that audit allocation-free paths. */
 int rb_device_alloc_count(int64_t* count);
 
 /* ||b - A x||_2 into norm_out[0] without allocating device memory.  No
@@ -431,11 +436,16 @@ int rb_adjoint_solve(rb_csr A, rb_amg ml, rb_vec lambda, rb_vec g, double tol, i
  * (rb_batch_offsets gives the first row of each). */
 int rb_batch_setup(int n_sys, const rb_csr* mats, const rb_amg_opts* opts, rb_batch* out);
 int rb_batch_destroy(rb_batch B);
-/* number of systems, total rows, levels of the packed hierarchy */
+/* number of systems, total rows, levels of the deepest system's hierarchy */
 int rb_batch_info(rb_batch B, int* n_sys, int64_t* total_rows, int* levels);
 /* offsets[n_sys + 1] (first row of each system, then the total) and the
  * levels of each system's own hierarchy (levels[n_sys]); either may be NULL */
 int rb_batch_offsets(rb_batch B, int64_t* offsets, int* levels);
+/* The levels of each system that the packed cycle keeps (cuts[n_sys]): the
+ * last of them is solved by a dense product, the system's coarsest or the
+ * level from which its cycle was made one product.  The packed hierarchy has
+ * as many levels as the largest. */
+int rb_batch_cuts(rb_batch B, int* cuts);
 /* x = M b: one V-cycle of every system from a zero guess */
 int rb_batch_cycle(rb_batch B, rb_vec x, rb_vec b);
 /* Preconditioned CG per system in true-residual mode; iters[n_sys] and

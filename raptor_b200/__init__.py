@@ -749,6 +749,13 @@ class ParMultilevel:
         check(lib().rb_amg_tail_info(self.h, C.byref(f), C.byref(c)))
         return f.value, c.value
 
+    def dense_info(self):
+        """(level from which the rest of the cycle is one dense product or -1,
+        that level's rows)."""
+        f, n = C.c_int(), C.c_int()
+        check(lib().rb_amg_dense_info(self.h, C.byref(f), C.byref(n)))
+        return f.value, n.value
+
     def print_hierarchy(self):
         print("Num Levels = %d" % self.num_levels)
         print("A\tNRow\tNCol\tNNZ")
@@ -821,6 +828,14 @@ class Batch:
 
     def cycle(self, x, b):
         check(lib().rb_batch_cycle(self.h, x.h, b.h))
+
+    @property
+    def cuts(self):
+        """Levels of each system that the packed cycle keeps; the last of
+        them is solved by a dense product."""
+        c = np.zeros(self.n_sys, np.int32)
+        check(lib().rb_batch_cuts(self.h, c.ctypes.data))
+        return c
 
     @property
     def host_waits(self):

@@ -136,6 +136,8 @@ SIGNATURES = {
     "rb_amg_level_lanes": (C.c_int, [_P, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "rb_amg_level_storage": (C.c_int, [_P, C.c_int, C.POINTER(C.c_int)]),
     "rb_amg_level_const_coef": (C.c_int, [_P, C.c_int, C.POINTER(C.c_int)]),
+    "rb_amg_dense_info": (C.c_int, [_P, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
+    "rb_batch_cuts": (C.c_int, [_P, _P]),
     "rb_amg_tail_info": (C.c_int, [_P, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "rb_amg_level_fused_first": (C.c_int, [_P, C.c_int, C.POINTER(C.c_int)]),
     "rb_amg_tail_timings": (C.c_int, [_P, _D, C.c_int, C.POINTER(C.c_int)]),

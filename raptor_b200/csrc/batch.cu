@@ -1074,7 +1074,8 @@ void batch_destroy(rb_batch_s* B) { delete B; }
 int batch_num_systems(const rb_batch_s* B) { return B->b.n_sys; }
 long long batch_offset(const rb_batch_s* B, int s) { return B->b.off[0][s]; }
 int batch_levels(const rb_batch_s* B, int s) { return B->b.depth[s]; }
-int batch_packed_levels(const rb_batch_s* B) { return B->b.max_depth; }
+int batch_cut(const rb_batch_s* B, int s) { return B->b.cut[s]; }
+int batch_max_levels(const rb_batch_s* B) { return B->b.max_depth; }
 void batch_cycle(rb_batch_s* B, double* x, const double* b) {
     Batch& T = B->b;
     char key[96];

@@ -1082,6 +1082,16 @@ int rb_amg_tail_info(rb_amg ml, int* start_level, int* ctas) {
     });
 }
 
+int rb_amg_dense_info(rb_amg ml, int* start_level, int* rows) {
+    return guarded([&]() -> int {
+        NEED(ml); NEED(start_level); NEED(rows);
+        const int f = ml->h.dense_from;
+        *start_level = f;
+        *rows = f >= 0 ? ml->h.master[f].A->n_rows : 0;
+        return RB_OK;
+    });
+}
+
 int rb_amg_tail_timings(rb_amg ml, double* ms, int cap, int* count) {
     return guarded([&]() -> int {
         NEED(ml); NEED(count);
@@ -1188,7 +1198,7 @@ int rb_batch_info(rb_batch B, int* n_sys, int64_t* total_rows, int* levels) {
         const int n = batch_num_systems(B);
         if (n_sys) *n_sys = n;
         if (total_rows) *total_rows = batch_offset(B, n);
-        if (levels) *levels = batch_packed_levels(B);
+        if (levels) *levels = batch_max_levels(B);
         return RB_OK;
     });
 }
@@ -1201,6 +1211,14 @@ int rb_batch_offsets(rb_batch B, int64_t* offsets, int* levels) {
             if (offsets) offsets[s] = batch_offset(B, s);
         for (int s = 0; s < n; s++)
             if (levels) levels[s] = batch_levels(B, s);
+        return RB_OK;
+    });
+}
+
+int rb_batch_cuts(rb_batch B, int* cuts) {
+    return guarded([&]() -> int {
+        NEED(B); NEED(cuts);
+        for (int s = 0; s < batch_num_systems(B); s++) cuts[s] = batch_cut(B, s);
         return RB_OK;
     });
 }

@@ -26,6 +26,34 @@ def make(prec, fuse, relax, compat=0):
 SETS = {"mixed": [5, 7, 13, 40, 90], "one": [64], "many": [60, 64, 68, 72] * 10}
 
 
+def expected_cuts(mats, prec, fuse, relax, compat):
+    """The size rule: down to the first level of at most 1024 rows, halved
+    until the matrices (FP64, rows padded to 16 bytes) fit 32 MB."""
+    sizes = []
+    for A in mats:
+        ml = make(prec, 0, relax, compat)
+        ml.setup(A)
+        sizes.append([ml.level_info(l)[0] for l in range(ml.num_levels)])
+    depth = [len(s) for s in sizes]
+    if fuse == 0 or relax == rb.SOR:
+        return depth
+    cap = 1024
+    while cap >= 64:
+        cuts = []
+        for s in sizes:
+            c = len(s)
+            for l in range(len(s) - 2, 0, -1):
+                if s[l] > cap:
+                    break
+                c = l + 1
+            cuts.append(c)
+        if sum(s[c - 1] * (s[c - 1] + 1 & ~1) * 8 for s, c in zip(sizes, cuts)) <= 32 << 20:
+            assert cuts != depth
+            return cuts
+        cap //= 2
+    return depth
+
+
 @pytest.mark.parametrize("prec", [rb.FP64, rb.FP32], ids=["fp64", "fp32"])
 @pytest.mark.parametrize("sides", sorted(SETS))
 @pytest.mark.parametrize("relax,compat", [(rb.L1Jacobi, 0), (rb.Jacobi, 1), (rb.SOR, 0)],
@@ -36,6 +64,7 @@ def test_batch_cycle_with_and_without_the_cut(sides, prec, relax, compat):
     got, levels = [], []
     for fuse in (0, 1):
         B = rb.Batch(mats, make(prec, fuse, relax, compat))
+        assert list(B.cuts) == expected_cuts(mats, prec, fuse, relax, compat)
         b = rb.ParVector(B.total_rows, values=np.random.default_rng(3).uniform(-1, 1, B.total_rows))
         x = rb.ParVector(B.total_rows)
         B.cycle(x, b)
