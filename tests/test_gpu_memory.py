@@ -21,8 +21,9 @@ def _device():
     rb.init(0)
 
 
-# 1 GiB arrays are the driver's own, 32 MiB ones the pool's, which keeps 2 GiB
-@pytest.mark.parametrize("log2n, kept", [(27, 0), (22, 2 << 30)])
+# 1 GiB arrays are the driver's own, 32 MiB ones cut from slabs, of which 1 GiB
+# is kept
+@pytest.mark.parametrize("log2n, kept", [(27, 0), (22, 1 << 30)])
 def test_freed_memory_is_given_back_above_the_bound(log2n, kept):
     rb.ParVector(1)
     rb.synchronize()
@@ -36,6 +37,26 @@ def test_freed_memory_is_given_back_above_the_bound(log2n, kept):
     rb.synchronize()
     # (and the driver's own granularity)
     assert torch.cuda.mem_get_info()[0] > before - kept - (256 << 20)
+
+
+def test_the_pool_keeps_at_most_2_gib():
+    """Block matrices of 32 MiB (their addresses are not given out: pool
+    memory), with a handle alive throughout, so that nothing else is given
+    back."""
+    b, nnz = 16, (4 << 20) // 256
+    vals = np.ones((nnz, b, b))
+    rowptr, cols = np.arange(nnz + 1, dtype=np.int32), np.zeros(nnz, np.int32)
+    alive = rb.ParVector(1)
+    rb.synchronize()
+    gc.collect()
+    before = torch.cuda.mem_get_info()[0]
+    big = [rb.BSRMatrix.from_arrays(nnz, 1, b, b, rowptr, cols, vals) for _ in range(112)]   # 3.5 GiB
+    assert torch.cuda.mem_get_info()[0] < before - (2 << 30)
+    del big
+    gc.collect()
+    rb.synchronize()
+    assert torch.cuda.mem_get_info()[0] > before - (2 << 30) - (256 << 20)
+    del alive
 
 
 def _ipc_capable(ptr):
