@@ -231,15 +231,27 @@ def cycle_bytes(ml, vbytes):
     (rows+1)i.  Pre-smooth from a zero guess reads b and the inverse diagonal
     and writes x (3nv), then the residual B_A + 3nv; where the level runs the
     two as one pass (level_fused_first) that pass is B_A + 4nv (b, D^-1 in,
-    x, r out); restriction B_R + n v + n_c v; prolongation B_P + (2n + n_c) v;
-    post-smooth B_A + 4nv (x, b, D^-1 in, x out).  Coarsest level: the dense
-    inverse product (n_c^2 8 bytes)."""
+    x, r out), and below level 0 the restriction from above writes the sweep;
+    restriction B_R + n v + n_c v (3 n_c v with the sweep: D^-1 in, x out);
+    prolongation B_P + (2n + n_c) v; post-smooth B_A + 4nv (x, b, D^-1 in, x
+    out).  From the level that starts the dense bottom (dense_info) down, one
+    product with its FP64 matrix (8 n^2 + 2nv); without it the coarsest level's
+    dense inverse product (n_c^2 8 bytes)."""
     L = ml.num_levels
     tot = 0.0
     per = []
+    dense, tail = ml.dense_info()[0], ml.tail_info()[0]
+
+    def swept(l):
+        return 0 < l < L - 1 and l != dense and l != tail and not ml.level_fused_first(l)
+
     for l in range(L):
         n, z, p = ml.level_info(l)
-        if l == L - 1:
+        if 0 <= dense < l:
+            b = 0.0
+        elif l == dense:
+            b = 8.0 * n * n + 2 * n * vbytes
+        elif l == L - 1:
             b = 1.0 * n * n * 8
         else:
             nc = ml.level_info(l + 1)[0]
@@ -249,8 +261,8 @@ def cycle_bytes(ml, vbytes):
             if ml.level_fused_first(l):
                 first = BA + 4 * n * vbytes
             else:
-                first = (3 * n * vbytes) + (BA + 3 * n * vbytes)
-            b = first + (BR + n * vbytes + nc * vbytes) + \
+                first = (0 if swept(l) else 3 * n * vbytes) + (BA + 3 * n * vbytes)
+            b = first + (BR + n * vbytes + (3 if swept(l + 1) else 1) * nc * vbytes) + \
                 (BP + (2 * n + nc) * vbytes) + (BA + 4 * n * vbytes)
         per.append(b)
         tot += b
@@ -767,7 +779,7 @@ def run_b200(args, rank, world, local):
         "method": {"smoother": "L1-Jacobi, 1 pre- and 1 post-sweep",
                    "cycle": "V-cycle in FP32 (hierarchy values FP32, int32 indices)",
                    "outer": "PCG in FP64, stopping on the true relative residual",
-                   "coarse": "FP64 LU of A_c^T (explicit inverse product)"},
+                   "coarse": "FP64 LU of A_c^T, its inverse applied in the bottom levels' dense FP64 product"},
         "iters": iters32[-1], "final_rel_res": rel32, "setup_s": setup32,
         "vcycle": {"ms": cyc_ms, "alg_bytes": cbytes_pc,
                    "gbs": cbytes_pc / (cyc_ms * 1e-3) / 1e9,
@@ -777,6 +789,7 @@ def run_b200(args, rank, world, local):
                    "alg_bytes_per_level": per_level,
                    "first_sweep_fused": [ml32.level_fused_first(l)
                                          for l in range(ml32.num_levels - 1)],
+                   "dense_bottom": dict(zip(("start_level", "rows"), ml32.dense_info())),
                    "tail": dict(zip(("start_level", "ctas"), ml32.tail_info()),
                                 cycle_ms_by_start=ml32.tail_timings()),
                    "levels": [ml32.level_info(l) for l in range(ml32.num_levels)],
