@@ -69,6 +69,15 @@ constexpr int kMaxDevices = 64;
 std::mutex g_pool_mu;
 cudaMemPool_t g_pools[kMaxDevices] = {};
 thread_local int t_handle_release = 0, t_handle_memory = 0;
+thread_local bool t_not_idle = false;   // a HandleRelease that could not wait
+// Memory freed while waiting was refused (a stream capture in progress, say
+// when a garbage collector runs in it): freed by the next HandleRelease that
+// could wait.
+std::mutex g_late_mu;
+std::vector<std::pair<void*, Mem>>& late_frees() {
+    static auto* v = new std::vector<std::pair<void*, Mem>>();
+    return *v;
+}
 std::atomic<long long> g_live{0};   // arrays of DevArrays
 std::mutex g_heap_mu;
 HandleHeap* heaps() {
@@ -180,8 +189,15 @@ void device_free(void* p, Mem kind) noexcept {
     const bool pooled = kind == Mem::kPool;
     cudaError_t e = cudaErrorUnknown;
     --g_live;
+    if (t_handle_release > 0 ? t_not_idle
+                             : kind == Mem::kHandle && cudaDeviceSynchronize() != cudaSuccess) {
+        (void)cudaGetLastError();
+        std::lock_guard<std::mutex> lock(g_late_mu);
+        late_frees().emplace_back(p, kind);
+        ++g_live;
+        return;
+    }
     if (kind == Mem::kHandle) {
-        if (t_handle_release == 0 && cudaDeviceSynchronize() != cudaSuccess) (void)cudaGetLastError();
         std::lock_guard<std::mutex> lock(g_heap_mu);
         for (int d = 0; d < kMaxDevices; d++)
             if (heaps()[d].owns(p)) {
@@ -211,13 +227,22 @@ void device_free(void* p, Mem kind) noexcept {
 }
 
 HandleRelease::HandleRelease() {
-    // (an error, such as a capture in progress elsewhere, leaves the frees to
-    // stream order on the library's own stream)
-    if (t_handle_release == 0 && cudaDeviceSynchronize() != cudaSuccess) (void)cudaGetLastError();
-    ++t_handle_release;
+    if (t_handle_release++ > 0) return;
+    t_not_idle = cudaDeviceSynchronize() != cudaSuccess;
+    if (t_not_idle) {
+        (void)cudaGetLastError();
+        return;
+    }
+    std::vector<std::pair<void*, Mem>> late;
+    {
+        std::lock_guard<std::mutex> lock(g_late_mu);
+        late.swap(late_frees());
+    }
+    for (auto& f : late) device_free(f.first, f.second);
 }
 HandleRelease::~HandleRelease() {
-    if (--t_handle_release > 0 || g_live != 0) return;
+    if (--t_handle_release > 0) return;
+    if (t_not_idle || g_live != 0) return;
     try {
         give_back(kIdleKeep, kIdleSlabs);
     } catch (const std::exception&) {   // no device any more, at process exit

@@ -162,6 +162,41 @@ def test_workspaces_replaced_while_another_stream_uses_them():
         np.testing.assert_allclose(X[k].numpy(), want[k], rtol=1e-12, atol=1e-14)
 
 
+def test_memory_freed_in_a_capture_is_not_reused_under_pending_reads():
+    """Waiting for the device is refused while a stream capture is in progress
+    (a garbage collector may run in one): the memory stays taken until a
+    later release could wait."""
+    from cuda.bindings import runtime
+
+    n = 1 << 22
+    v = rb.ParVector(n, values=np.full(n, 3.0))
+    t, at = v.torch_view(), v.device_ptr()
+    acc = torch.zeros(n, dtype=torch.float64, device="cuda")
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    err, c = runtime.cudaStreamCreateWithFlags(runtime.cudaStreamNonBlocking)
+    assert int(err) == 0
+    with torch.cuda.stream(side):
+        for _ in range(200):
+            acc += t
+    (err,) = runtime.cudaStreamBeginCapture(c, runtime.cudaStreamCaptureMode.cudaStreamCaptureModeGlobal)
+    assert int(err) == 0
+    del t, v
+    gc.collect()
+    runtime.cudaStreamEndCapture(c)      # (the wait that was tried ended it)
+    runtime.cudaGetLastError()
+    new = [rb.ParVector(n, values=np.full(n, -7.0)) for _ in range(4)]
+    assert all(w.device_ptr() != at for w in new)
+    side.synchronize()
+    assert torch.all(acc == 600.0)
+    del new                              # the late free happens here
+    gc.collect()
+    runtime.cudaStreamDestroy(c)
+    # (more than the slabs keep free: one of them covers the place again)
+    again = [rb.ParVector(n) for _ in range(40)]
+    assert any(w.device_ptr() <= at < w.device_ptr() + 8 * n for w in again)
+
+
 def test_memory_goes_back_once_the_last_handle_is_gone():
     """A hierarchy and vectors of 1.5 GiB: with every handle destroyed at most
     384 MiB stay with the library, and after rb.trim() nothing but the
