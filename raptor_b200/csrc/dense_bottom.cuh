@@ -19,9 +19,9 @@
 // nearly singular operator its entries are dominated by the large multiple of
 // the near-null vector's projector, and rounded to FP32 they lose what the
 // cycle does to everything else (graph Laplacian + 1e-7 on 40^3: error off
-// the constant 2e-4, in FP64 8e-8).  With the 16 MB below it costs an FP32
-// cycle nothing (192^3 PCG 8.42 and 8.50 ms, 1024^2 12.6 and 12.2, runs of one
-// side 2.5% apart; 32 MB and its 2048 rows: 8.51 and 12.5).
+// the constant 2e-4, in FP64 8e-8).  On the same schedules an FP32 cycle
+// takes as long with either (192^3 478.3 and 478.6 us, 1024^2 143.4 and 143.3),
+// k = 8 columns of 96^3 1.5% longer (11.5 -> 11.7 ms a solve).
 #pragma once
 
 #include "rb_common.cuh"
